@@ -34,6 +34,9 @@ struct DenseInst {
 constexpr u32 kDenseFlagLevels = 1;   // a row went deeper than the level arrays hold
 constexpr u32 kDenseFlagRange = 2;    // a value outside its row's instance range
 constexpr u64 kDenseMaxN = 65536;     // values per instance (3 rows of bits in shared memory)
+// not an edge: the self-loop of an instance's value 0, which never adds a tuple (its target
+// is known as soon as its source is on a frontier)
+constexpr u32 kNoEdge = 0;
 
 struct DenseArgs {
     const DenseInst* inst;       // n_inst entries (1 without instances)
@@ -41,20 +44,25 @@ struct DenseArgs {
     u32 n_inst;
     u64 rows;                    // rows 0 .. rows-1 are the values of the union
     u32* known;                  // known tuples; after the closure pass: the new ones
-    u32* delta0;                 // the SCC's initial delta
+    u32* delta0;                 // the SCC's initial delta (the same matrix when R's full version is empty)
     int bits;                    // packed column width
     const u64* s_keys;           // S full rows, sorted
     const u64* s_csr;            // S rows with column 0 == v: [s_csr[v], s_csr[v + 1])
-    u32* s_local;                // per S row: column 1 minus the instance base of its column 0
+    u32* s_edge;                 // per S row: its columns minus its instance's base, column 0 in the upper half
     u64* row_new;                // per row: new tuples
     u64* level_total;            // per iteration: new tuples
     u64* inst_level;             // [iteration][instance] new tuples, or null
     u64 level_cap;
-    u64* inst_init;              // per instance: tuples of the initial delta
     u64* counters;               // [0], [2..4] chunks taken (per kernel shape), [1] join candidates (S rows visited),
                                  // [5] 1 + the first key found outside its instance, [6] its relation (1: R, 2: S)
     u32* flags;
 };
+
+// S rows of value y (the edges a search visits when it reaches y)
+__device__ __forceinline__ u64 row_edges(const DenseArgs& a, u64 y)
+{
+    return y < a.rows ? a.s_csr[y + 1] - a.s_csr[y] : 0;
+}
 
 __device__ __forceinline__ u32 dense_instance(const DenseArgs& a, u64 v)
 {
@@ -86,16 +94,13 @@ __global__ void __launch_bounds__(kThreads) dense_load_kernel(DenseArgs a, const
         const u64 w = d.word_off + r * d.words + (c >> 5);
         const u32 bit = 1u << (c & 31);
         atomicOr(&a.known[w], bit);
-        if (i >= n_full) {
-            atomicOr(&a.delta0[w], bit);
-            atomicAdd((unsigned long long*)&a.inst_init[inst], 1ull);
-        }
+        if (i >= n_full && a.delta0 != a.known) atomicOr(&a.delta0[w], bit);
     }
 }
 
-// S's column 1 as instance-local values, once per SCC (the search's inner loop
-// then reads 4 bytes per edge and compares once); a value outside its row's
-// instance is stored as 0xffffffff, which the search rejects.
+// S's rows as instance-local pairs, once per SCC (the searches' inner loops then read
+// 4 bytes per edge); a row with a value outside its instance is stored as kNoEdge (the
+// run fails).
 __global__ void __launch_bounds__(kThreads) dense_local_kernel(DenseArgs a, u64 n)
 {
     for (u64 j = (u64)blockIdx.x * kThreads + threadIdx.x; j < n; j += (u64)gridDim.x * kThreads) {
@@ -104,10 +109,10 @@ __global__ void __launch_bounds__(kThreads) dense_local_kernel(DenseArgs a, u64 
         const DenseInst d = a.inst[dense_instance(a, y)];
         const u64 zl = z - d.base;
         if (zl >= d.n || y - d.base >= d.n) {
-            a.s_local[j] = 0xffffffffu;
+            a.s_edge[j] = kNoEdge;
             dense_range_error(a, k, 2);
         } else {
-            a.s_local[j] = (u32)zl;
+            a.s_edge[j] = (u32)((y - d.base) << 16 | zl);
         }
     }
 }
@@ -119,7 +124,6 @@ struct DenseChunk {
     u32 count;
 };
 
-constexpr u32 kDenseWarpWords = 512;  // instances of at most 16384 values: one warp per row
 constexpr int kDenseLevels = 64;      // levels counted in shared memory per chunk (deeper ones directly)
 
 // A level's new-tuple count of a row: into the chunk's shared counters, or
@@ -152,9 +156,9 @@ __device__ __forceinline__ void dense_flush_levels(const DenseArgs& a, u64* lvl,
     }
 }
 
-// Rows of instances with more than kDenseWarpWords words: one CTA per row,
-// chunks taken from a device counter; the row's whole search in shared
-// memory.  Dynamic shared memory: 3 * wmax u32.
+// Rows of instances with more than kMsMaxN values: one CTA per row, chunks taken from
+// a device counter; the row's whole search in shared memory.  Dynamic shared memory:
+// 3 * wmax u32.
 __global__ void __launch_bounds__(kThreads) dense_closure_kernel(DenseArgs a, u32 wmax, const DenseChunk* __restrict__ chunks,
                                                                  u64 n_chunks, u64* __restrict__ chunk_ctr)
 {
@@ -201,8 +205,7 @@ __global__ void __launch_bounds__(kThreads) dense_closure_kernel(DenseArgs a, u3
                         const u64 s = a.s_csr[y], e = a.s_csr[y + 1];
                         relax += e - s;
                         for (u64 j = s; j < e; j++) {
-                            const u32 z = a.s_local[j];
-                            if (z >= (u32)d.n) continue;   // flagged by dense_local_kernel
+                            const u32 z = a.s_edge[j] & 0xffffu;
                             const u32 bit = 1u << (z & 31);
                             if (!(known[z >> 5] & bit)) atomicOr(&next[z >> 5], bit);
                         }
@@ -235,105 +238,219 @@ __global__ void __launch_bounds__(kThreads) dense_closure_kernel(DenseArgs a, u3
     if (threadIdx.x == 0 && relax) atomicAdd((unsigned long long*)&a.counters[1], (unsigned long long)relax);
 }
 
-// Rows of instances of at most 32 * MW words (MW * 1024 values): one warp per
-// row, lane l owning words l, l + 32, ... (its frontier words in registers,
-// the row's known and next-level bits in the warp's shared memory); no block
-// barriers, so rows with small searches cost little.  Chunks are taken per
-// warp from a device counter.
-template <int MW>
-__global__ void __launch_bounds__(kThreads) dense_closure_warp_kernel(DenseArgs a, const DenseChunk* __restrict__ chunks,
-                                                                      u64 n_chunks, u64* __restrict__ chunk_ctr)
+// 32 x 32 bit transpose across a warp: bit r of lane l's result is bit l of lane r's word.
+__device__ __forceinline__ u32 warp_transpose32(u32 x)
 {
-    constexpr int WW = 32 * MW;   // words a warp's row may have
-    __shared__ u32 s_known[kWarps][WW];
-    __shared__ u32 s_next[kWarps][WW];
-    __shared__ u64 s_lvl[kWarps][kDenseLevels];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 16, k = 0; j; j >>= 1, k++) {
+        const u32 m = k == 0 ? 0x0000ffffu : k == 1 ? 0x00ff00ffu : k == 2 ? 0x0f0f0f0fu : k == 3 ? 0x33333333u : 0x55555555u;
+        const u32 y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+    }
+    return x;
+}
+
+// z to the end of a block's queue; called by the lanes that have one (any subset of a warp).
+__device__ __forceinline__ void queue_push(u16* q, u32* qn, u32 z)
+{
+    const u32 m = __activemask();
+    const u32 before = __popc(m & lanemask_lt());
+    u32 at = 0;
+    if (before == 0) at = atomicAdd(qn, (u32)__popc(m));
+    at = __shfl_sync(m, at, __ffs(m) - 1);
+    q[at + before] = (u16)z;
+}
+
+constexpr int kMsRows = 32;           // rows searched together: one bit each of a value's words
+constexpr u64 kMsMaxN = 19200;        // values per instance: three words of each fit an SM's shared memory
+constexpr u32 kMsSmemQueueN = 13824;  // ... with both queues beside them; above, the queues are in global memory
+
+// Rows of instances of at most kMsMaxN values: 32 rows of one instance at a time by one
+// CTA, their breadth-first searches run together.  Value z has one word each of known,
+// frontier and next bits, bit r for the group's row r; a level visits every value of the
+// frontier once for all the rows that reached it in that level, where a search per row
+// visits it once for each row: in a dense closure (n = 14,336, out-degree 2, 26 levels) 32
+// rows meet each value in 7 levels.  A level with a wide frontier (1/kMsSweep of the
+// values) sweeps the instance's edge list, every lane an edge -- each warp's frontier words
+// are neighbours in shared memory, and no lane waits for another's longer list; a
+// narrow one follows the queue of its values (its edge ranges and edges are a chain of L2
+// round trips: with 1/8, 1/16, 1/32 and 1/64 of the values as the line between the two, a wave
+// of 64 graphs ran its fixed point in 7.13, 6.98, 6.91 and 6.80 ms, and always queueing took
+// 11.5).  Bound by instruction issue and shared-memory conflicts of the random known / next
+// words.  Measured against one warp or CTA per row: n = 16,384, out-degree 2, 3.52 -> 0.97 ms;
+// n = 2,000, 0.24 -> 0.09 ms; the wave's searches 10.0 -> 4.9 ms.
+// Dynamic shared memory: 3 * nmax u32, then (gqueue null) 2 * nmax u16.
+constexpr u32 kMsSweep = 64;
+template <int T>
+__global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16* __restrict__ gqueue,
+                                                     const DenseChunk* __restrict__ chunks, u64 n_chunks,
+                                                     u64* __restrict__ chunk_ctr)
+{
+    extern __shared__ u32 dsm[];
+    u32* known = dsm;
+    u32* front = dsm + nmax;
+    u32* next = dsm + 2 * (u64)nmax;
+    u16* queue = gqueue ? gqueue + (u64)blockIdx.x * 2 * nmax : (u16*)(dsm + 3 * (u64)nmax);
+    __shared__ u64 s_chunk;
+    __shared__ u32 s_qn[2];
+    __shared__ u32 s_lvl[kDenseLevels];   // a chunk's counts stay below 32 * kMsMaxN
+    __shared__ u32 s_row[kMsRows];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    u32* known = s_known[warp];
-    u32* next = s_next[warp];
-    u64* lvl = s_lvl[warp];
-    for (int i = lane; i < kDenseLevels; i += 32) lvl[i] = 0;
     u64 relax = 0;
     for (;;) {
-        u64 c = 0;
-        if (lane == 0) c = atomicAdd((unsigned long long*)chunk_ctr, 1ull);
-        c = __shfl_sync(0xffffffffu, c, 0);
+        if (threadIdx.x == 0) {
+            s_chunk = atomicAdd((unsigned long long*)chunk_ctr, 1ull);
+            s_qn[0] = s_qn[1] = 0;
+        }
+        for (int i = threadIdx.x; i < kDenseLevels; i += T) s_lvl[i] = 0;
+        if (threadIdx.x < kMsRows) s_row[threadIdx.x] = 0;
+        __syncthreads();
+        const u64 c = s_chunk;
         if (c >= n_chunks) break;
         const DenseChunk ch = chunks[c];
         const DenseInst d = a.inst[ch.inst];
-        const u32 W = (u32)d.words;   // <= WW by the host's dispatch
-        for (u32 k = 0; k < ch.count; k++) {
-            const u64 row = ch.first_row + k;
-            u32* krow = a.known + d.word_off + (row - d.base) * d.words;
-            const u32* drow = a.delta0 + d.word_off + (row - d.base) * d.words;
-            u32 fr[MW];
-            bool any = false;
-#pragma unroll
-            for (int q = 0; q < MW; q++) {
-                const u32 w = (u32)(q * 32 + lane);
-                fr[q] = 0;
-                if (w < W) {
-                    known[w] = krow[w];
-                    next[w] = 0;
-                    fr[q] = drow[w];
-                    any |= fr[q] != 0;
-                }
-            }
-            __syncwarp();
-            if (!__any_sync(0xffffffffu, any)) continue;
-            u64 level = 0, total = 0;
-            for (;;) {
-#pragma unroll
-                for (int q = 0; q < MW; q++) {
-                    u32 f = fr[q];
-                    const u64 w = (u64)(q * 32 + lane);
-                    while (f) {
-                        const u32 b = __ffs(f) - 1;
-                        f &= f - 1;
-                        const u64 y = d.base + w * 32 + b;
-                        const u64 s = a.s_csr[y], e = a.s_csr[y + 1];
-                        relax += e - s;
-                        for (u64 j = s; j < e; j++) {
-                            const u32 z = a.s_local[j];
-                            if (z >= (u32)d.n) continue;   // flagged by dense_local_kernel
-                            const u32 bit = 1u << (z & 31);
-                            if (!(known[z >> 5] & bit)) atomicOr(&next[z >> 5], bit);
-                        }
-                    }
-                }
-                __syncwarp();
-                u32 cnt = 0;
-#pragma unroll
-                for (int q = 0; q < MW; q++) {
-                    const u32 w = (u32)(q * 32 + lane);
-                    fr[q] = 0;
-                    if (w < W) {
-                        const u32 nw = next[w] & ~known[w];
-                        next[w] = 0;
-                        known[w] |= nw;
-                        fr[q] = nw;
-                        cnt += __popc(nw);
-                    }
-                }
-                cnt = __reduce_add_sync(0xffffffffu, cnt);
-                __syncwarp();
-                if (cnt == 0) break;
-                if (lane == 0) dense_count_level(a, lvl, level, ch.inst, cnt);
-                total += cnt;
-                level++;
-            }
-            // the row's new tuples replace its known bits in global memory
-#pragma unroll
-            for (int q = 0; q < MW; q++) {
-                const u32 w = (u32)(q * 32 + lane);
-                if (w < W) krow[w] = known[w] & ~krow[w];
-            }
-            if (lane == 0) a.row_new[row] = total;
-            __syncwarp();
+        const u32 W = (u32)d.words;
+        const u64 w0 = d.word_off + (ch.first_row - d.base) * d.words;
+        u32* krow = a.known + w0 + (u64)lane * d.words;      // lane r: row r of the group
+        const u32* drow = a.delta0 + w0 + (u64)lane * d.words;
+        const bool own = lane < (int)ch.count;
+        const u32 n = (u32)d.n;
+        const u64 e0 = a.s_csr[d.base], e1 = a.s_csr[min(d.base + d.n, a.rows)];   // the instance's edges
+        for (u32 w = warp; w < W; w += T / 32) {
+            const u32 kw = warp_transpose32(own ? krow[w] : 0u);
+            const u32 fw = drow == krow ? kw : warp_transpose32(own ? drow[w] : 0u);
+            const u32 z = w * 32 + lane;
+            known[z] = kw;
+            front[z] = fw;
+            next[z] = 0;
+            if (fw) queue_push(queue, &s_qn[0], z);
+            if (z < n) relax += row_edges(a, d.base + z) * (u64)(long long)(__popc(fw) - __popc(kw));
         }
-        __syncwarp();
-        dense_flush_levels(a, lvl, ch.inst, lane, 32);
-        __syncwarp();
+        __syncthreads();
+        u32 cur = 0, qn = s_qn[0];
+        bool queued = true;   // queue `cur` lists the frontier's values
+        for (u64 level = 0; qn; level++) {
+            const u16* q = queue + (cur ? nmax : 0);
+            u16* qnext = queue + (cur ? 0 : nmax);
+            u32 cnt = 0;
+            if (qn >= n / kMsSweep) {
+                queued = false;
+                for (u64 j = (e0 & ~3ull) + 4 * threadIdx.x; j < e1; j += 4 * T) {
+                    u32 edge[4];
+                    *(uint4*)edge = *(const uint4*)(a.s_edge + j);
+                    if (j < e0 || j + 4 > e1) {   // another instance's edges
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            if (j + k < e0 || j + k >= e1) edge[k] = kNoEdge;
+                    }
+                    u32 fr[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) fr[k] = front[edge[k] >> 16];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (!fr[k]) continue;
+                        const u32 z = edge[k] & 0xffffu;
+                        const u32 nb = fr[k] & ~known[z];
+                        if (nb) atomicOr(&next[z], nb);
+                    }
+                }
+                __syncthreads();
+                u32 some = 0;   // values of the new frontier
+                for (u32 z = 4 * threadIdx.x; z < W * 32; z += 4 * T) {
+                    const uint4 f = *(const uint4*)(next + z);
+                    *(uint4*)(front + z) = f;
+                    if (!(f.x | f.y | f.z | f.w)) continue;
+                    *(uint4*)(next + z) = make_uint4(0, 0, 0, 0);
+                    uint4 k = *(const uint4*)(known + z);
+                    k.x |= f.x;
+                    k.y |= f.y;
+                    k.z |= f.z;
+                    k.w |= f.w;
+                    *(uint4*)(known + z) = k;
+                    cnt += __popc(f.x) + __popc(f.y) + __popc(f.z) + __popc(f.w);
+                    some += (f.x != 0) + (f.y != 0) + (f.z != 0) + (f.w != 0);
+                }
+                some = __reduce_add_sync(0xffffffffu, some);
+                if (lane == 0 && some) atomicAdd(&s_qn[cur ^ 1], some);
+            } else {
+                if (!queued) {   // a sweep counted the frontier's values: list them
+                    __syncthreads();   // every thread has read the count
+                    if (threadIdx.x == 0) s_qn[cur] = 0;
+                    __syncthreads();
+                    for (u32 z = threadIdx.x; z < W * 32; z += T)
+                        if (front[z]) queue_push(queue + (cur ? nmax : 0), &s_qn[cur], z);
+                    queued = true;
+                    __syncthreads();
+                }
+                for (u32 i = threadIdx.x; i < qn; i += T) {
+                    const u32 y = q[i];
+                    const u32 f = front[y];
+                    front[y] = 0;
+                    const u64 s = a.s_csr[d.base + y], e = a.s_csr[d.base + y + 1];
+                    for (u64 j = s; j < e; j++) {
+                        const u32 z = a.s_edge[j] & 0xffffu;
+                        const u32 nb = f & ~known[z];
+                        if (nb && atomicOr(&next[z], nb) == 0) queue_push(qnext, &s_qn[cur ^ 1], z);
+                    }
+                }
+                __syncthreads();
+                const u32 qnew = s_qn[cur ^ 1];
+                for (u32 i = threadIdx.x; i < qnew; i += T) {
+                    const u32 z = qnext[i];
+                    const u32 f = next[z];
+                    next[z] = 0;
+                    known[z] |= f;
+                    front[z] = f;
+                    cnt += __popc(f);
+                }
+            }
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0 && cnt) {
+                if (level < (u64)kDenseLevels) {
+                    atomicAdd(&s_lvl[level], cnt);
+                } else if (level < a.level_cap) {
+                    atomicAdd((unsigned long long*)&a.level_total[level], (unsigned long long)cnt);
+                    if (a.inst_level)
+                        atomicAdd((unsigned long long*)&a.inst_level[level * a.n_inst + ch.inst],
+                                  (unsigned long long)cnt);
+                } else {
+                    atomicOr(a.flags, kDenseFlagLevels);
+                }
+            }
+            if (threadIdx.x == 0) s_qn[cur] = 0;
+            __syncthreads();
+            cur ^= 1;
+            qn = s_qn[cur];
+        }
+        // the rows' new tuples replace their known bits in global memory
+        u32 rcnt = 0;
+        for (u32 w = warp; w < W; w += T / 32) {
+            const u32 z = w * 32 + lane;
+            const u32 kz = known[z];
+            const u32 t = warp_transpose32(kz);
+            if (z < n) relax += row_edges(a, d.base + z) * (u64)__popc(kz);
+            if (own) {
+                const u32 nw = t & ~krow[w];
+                krow[w] = nw;
+                rcnt += __popc(nw);
+            }
+        }
+        if (rcnt) atomicAdd(&s_row[lane], rcnt);
+        __syncthreads();
+        if (threadIdx.x < ch.count) a.row_new[ch.first_row + threadIdx.x] = s_row[threadIdx.x];
+        for (int i = threadIdx.x; i < kDenseLevels; i += T) {
+            const u32 v = s_lvl[i];
+            if (!v) continue;
+            if ((u64)i < a.level_cap) {
+                atomicAdd((unsigned long long*)&a.level_total[i], (unsigned long long)v);
+                if (a.inst_level)
+                    atomicAdd((unsigned long long*)&a.inst_level[(u64)i * a.n_inst + ch.inst], (unsigned long long)v);
+            } else {
+                atomicOr(a.flags, kDenseFlagLevels);
+            }
+        }
+        __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1) relax += __shfl_xor_sync(0xffffffffu, relax, o);
     if (lane == 0 && relax) atomicAdd((unsigned long long*)&a.counters[1], (unsigned long long)relax);

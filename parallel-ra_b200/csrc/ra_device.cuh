@@ -15,6 +15,7 @@ namespace ra {
 typedef unsigned long long u64;
 typedef unsigned char u8;
 typedef unsigned int u32;
+typedef unsigned short u16;
 
 constexpr u64 kEmpty = ~0ull;          // empty hash slot / filtered candidate
 constexpr int kThreads = 256;          // block size of every engine kernel

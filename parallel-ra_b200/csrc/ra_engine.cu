@@ -2178,10 +2178,10 @@ struct DenseBufs {
     u64* level_total = nullptr;
     u64* counters = nullptr;
     u32* flags = nullptr;
-    u32* s_local = nullptr;
+    u32* s_edge = nullptr;
     DenseInst* inst = nullptr;
     DenseChunk* chunks = nullptr;
-    u64* inst_init = nullptr;
+    u16* queue = nullptr;
     explicit DenseBufs(ra_program* pp) : p(pp) {}
     ~DenseBufs()
     {
@@ -2192,10 +2192,10 @@ struct DenseBufs {
         dev_free(p, &level_total);
         dev_free(p, &counters);
         dev_free(p, &flags);
-        dev_free(p, &s_local);
+        dev_free(p, &s_edge);
         dev_free(p, &inst);
         dev_free(p, &chunks);
-        dev_free(p, &inst_init);
+        dev_free(p, &queue);
     }
 };
 
@@ -2284,21 +2284,28 @@ bool run_scc_dense(ra_program* p, Scc& s)
     if (2.0 * 4.0 * (double)words + 16.0 * (double)rows > p->tune.dense_max_bytes) return false;
 
     DenseBufs B(p);
+    const bool all_delta = R.full_n == 0;   // every stored tuple is in the initial delta: one matrix holds both
     dev_alloc(p, &B.known, words);
-    dev_alloc(p, &B.delta0, words);
+    if (!all_delta) dev_alloc(p, &B.delta0, words);
     dev_alloc(p, &B.row_new, rows);
     dev_alloc(p, &B.row_off, rows);
     dev_alloc(p, &B.counters, 8);
     dev_alloc(p, &B.flags, 1);
     dev_alloc(p, &B.inst, ninst);
-    dev_alloc(p, &B.inst_init, ninst);
-    constexpr int kShapes = 4;   // search kernels: warp per row with 1, 4, 16 words per lane; CTA per row
+    // the searches: 32 rows of an instance per CTA (dense_ms_kernel) in four shapes by the
+    // instance's values, or one row per CTA (dense_closure_kernel) above kMsMaxN values
+    constexpr int kShapes = 5;
+    const u64 ms_n[4] = {1024, 4096, kMsSmemQueueN, kMsMaxN};
+    typedef void (*DenseMs)(DenseArgs, u32, u16*, const DenseChunk*, u64, u64*);
+    const DenseMs ms_all[4] = {dense_ms_kernel<128>, dense_ms_kernel<256>, dense_ms_kernel<512>, dense_ms_kernel<1024>};
+    constexpr u64 kDenseSmemMax = 12 * kMsMaxN;   // 16 * kMsSmemQueueN is less
+    static_assert(16 * kMsSmemQueueN <= kDenseSmemMax && kDenseSmemMax <= 225u << 10, "dynamic shared memory of an SM");
     CK(cudaMemcpyAsync(B.inst, hi.data(), ninst * sizeof(DenseInst), cudaMemcpyHostToDevice, p->stream));
     const u64 *sk, *sv;
     u64 sn;
     version_rows(p, S, RA_FULL, &sk, &sv, &sn);
     const u64* scsr = version_csr(p, S, RA_FULL);
-    dev_alloc(p, &B.s_local, sn);
+    dev_alloc(p, &B.s_edge, (sn + 3) & ~3ull);   // read four at a time
     const u64 n_stored = R.full_n + R.delta_n;
     u64 level_cap = 256;
     std::vector<u64> hflags(2);
@@ -2310,28 +2317,26 @@ bool run_scc_dense(ra_program* p, Scc& s)
             CK(cudaMemsetAsync(p->dinst_new, 0, p->inst_rows_cap * p->n_inst * 8, p->stream));
         }
         CK(cudaMemsetAsync(B.known, 0, words * 4, p->stream));
-        CK(cudaMemsetAsync(B.delta0, 0, words * 4, p->stream));
+        if (!all_delta) CK(cudaMemsetAsync(B.delta0, 0, words * 4, p->stream));
         CK(cudaMemsetAsync(B.row_new, 0, rows * 8, p->stream));
         CK(cudaMemsetAsync(B.level_total, 0, level_cap * 8, p->stream));
         CK(cudaMemsetAsync(B.counters, 0, 8 * 8, p->stream));
         CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
-        CK(cudaMemsetAsync(B.inst_init, 0, ninst * 8, p->stream));
         DenseArgs a{};
         a.inst = B.inst;
         a.inst_base = p->n_inst ? p->dinst_base : nullptr;
         a.n_inst = ninst;
         a.rows = rows;
         a.known = B.known;
-        a.delta0 = B.delta0;
+        a.delta0 = all_delta ? B.known : B.delta0;
         a.bits = p->bits;
         a.s_keys = sk;
         a.s_csr = scsr;
-        a.s_local = B.s_local;
+        a.s_edge = B.s_edge;
         a.row_new = B.row_new;
         a.level_total = B.level_total;
         a.inst_level = p->n_inst ? p->dinst_new : nullptr;
         a.level_cap = p->n_inst ? std::min(level_cap, p->inst_rows_cap) : level_cap;
-        a.inst_init = B.inst_init;
         a.counters = B.counters;
         a.flags = B.flags;
         if (sn) {
@@ -2342,35 +2347,25 @@ bool run_scc_dense(ra_program* p, Scc& s)
             dense_load_kernel<<<grid_for(n_stored), kThreads, 0, p->stream>>>(a, R.keys, R.full_n, n_stored);
             LAUNCHED();
         }
-        // work: chunks of rows of one instance.  A row's search reaches about s * n values when the
-        // initial delta averages d > 1 tuples per row (s = 1 - exp(-d s), the giant component of a
-        // random graph), a handful otherwise.  Instances whose rows reach at most 1024 values (and
-        // of at most 16384 values) run one warp per row (words per lane 1, 4 or 16: three kernel
-        // shapes), with no block barriers; wider searches run one CTA per row.
-        std::vector<u64> init(ninst);
-        CK(cudaMemcpyAsync(init.data(), B.inst_init, ninst * 8, cudaMemcpyDeviceToHost, p->stream));
-        CK(cudaStreamSynchronize(p->stream));
+        // work: chunks of rows of one instance, the widest instances first
         auto shape_of = [&](u32 i) {
-            const u64 w = hi[i].words;
-            const double n = (double)hi[i].n, deg = (double)init[i] / n;
-            double sfrac = 0.0;
-            if (deg > 1.0) {
-                sfrac = 0.5;
-                for (int it = 0; it < 60; it++) sfrac = 1.0 - std::exp(-deg * sfrac);
-            }
-            if (w > 512 || (w > 32 && sfrac * n > 1024.0)) return 3;
-            return w <= 32 ? 0 : w <= 128 ? 1 : 2;
+            int sh = 0;
+            while (sh < 4 && hi[i].n > ms_n[sh]) sh++;
+            return sh;
         };
+        std::vector<u32> order(ninst);
+        for (u32 i = 0; i < ninst; i++) order[i] = i;
+        std::stable_sort(order.begin(), order.end(), [&](u32 x, u32 y) { return hi[x].n > hi[y].n; });
         std::vector<DenseChunk> chunks;
         u64 first[kShapes + 1] = {0};
-        u64 cta_wmax = 1;
+        u64 nmax[kShapes] = {0};
         for (int sh = 0; sh < kShapes; sh++) {
             first[sh] = chunks.size();
-            for (u32 i = 0; i < ninst; i++) {
+            for (u32 i : order) {
                 const DenseInst& di = hi[i];
                 if (shape_of(i) != sh || di.base >= rows) continue;
-                if (sh == 3) cta_wmax = std::max(cta_wmax, di.words);
-                const u64 cnt = std::min(di.n, rows - di.base), per = sh == 3 ? 4 : 8;
+                nmax[sh] = std::max(nmax[sh], (di.n + 31) / 32 * 32);
+                const u64 cnt = std::min(di.n, rows - di.base), per = sh == 4 ? 4 : kMsRows;
                 for (u64 r0 = 0; r0 < cnt; r0 += per)
                     chunks.push_back(DenseChunk{di.base + r0, i, (u32)std::min(per, cnt - r0)});
             }
@@ -2381,20 +2376,32 @@ bool run_scc_dense(ra_program* p, Scc& s)
         if (!chunks.empty())
             CK(cudaMemcpyAsync(B.chunks, chunks.data(), chunks.size() * sizeof(DenseChunk), cudaMemcpyHostToDevice,
                                p->stream));
-        const size_t smem = 3 * cta_wmax * sizeof(u32);
-        // grids: resident CTAs of each kernel, at most one warp (CTA) per chunk
-        auto resident = [&](const void* fn, size_t dyn) {
-            int per_sm = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, dyn));
-            return (u64)kSms * (u64)std::max(per_sm, 1);
-        };
-        const void* fns[kShapes] = {(const void*)dense_closure_warp_kernel<1>, (const void*)dense_closure_warp_kernel<4>,
-                                    (const void*)dense_closure_warp_kernel<16>, (const void*)dense_closure_kernel};
-        int grids[kShapes];
+        // grids: resident CTAs of each kernel, at most one per chunk
+        u64* ctr[kShapes] = {B.counters + 2, B.counters + 3, B.counters + 4, B.counters + 7, B.counters};
+        u64 nc[kShapes];
+        DenseMs fn[4] = {nullptr, nullptr, nullptr, nullptr};
+        size_t smem[kShapes];
+        int grids[kShapes], threads[kShapes];
         for (int sh = 0; sh < kShapes; sh++) {
-            const u64 n = first[sh + 1] - first[sh];
-            const u64 want = sh == 3 ? n : (n + kWarps - 1) / kWarps;
-            grids[sh] = (int)std::max<u64>(1, std::min(resident(fns[sh], sh == 3 ? smem : 0), want));
+            nc[sh] = first[sh + 1] - first[sh];
+            if (!nc[sh]) continue;
+            // threads per CTA: as many as its values when the chunks leave SMs idle, else several CTAs per SM
+            const bool few = nc[sh] <= (u64)kSms;
+            const int t = sh >= 2 ? 3 : sh == 1 ? (few ? 3 : 1) : (few ? (nmax[sh] > 256 ? 2 : 1) : 0);
+            threads[sh] = sh == 4 ? kThreads : 128 << t;
+            const void* k = (const void*)dense_closure_kernel;
+            if (sh < 4) k = (const void*)(fn[sh] = ms_all[t]);
+            smem[sh] = sh == 4 ? 3 * (nmax[sh] / 32) * sizeof(u32)
+                               : (3 * sizeof(u32) + (sh == 3 ? 0 : 2 * sizeof(u16))) * nmax[sh];
+            if (smem[sh] > 40u << 10)   // the most any launch of this kernel asks for (shapes share kernels)
+                CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmemMax));
+            int per_sm = 0;
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads[sh], smem[sh]));
+            grids[sh] = (int)std::max<u64>(1, std::min((u64)kSms * (u64)std::max(per_sm, 1), nc[sh]));
+        }
+        if (nc[3]) {
+            dev_free(p, &B.queue);
+            dev_alloc(p, &B.queue, (u64)grids[3] * 2 * nmax[3]);
         }
         cudaEvent_t ev[2] = {nullptr, nullptr};
         if (p->kernel_events) {
@@ -2402,18 +2409,13 @@ bool run_scc_dense(ra_program* p, Scc& s)
             CK(cudaEventCreate(&ev[1]));
             CK(cudaEventRecord(ev[0], p->stream));
         }
-        // one chunk counter per shape: counters[0] and [2] .. [4]
-        u64* ctr[kShapes] = {B.counters + 2, B.counters + 3, B.counters + 4, B.counters};
-        const u64 nc[kShapes] = {first[1] - first[0], first[2] - first[1], first[3] - first[2], first[4] - first[3]};
-        if (nc[0])
-            dense_closure_warp_kernel<1><<<grids[0], kThreads, 0, p->stream>>>(a, B.chunks + first[0], nc[0], ctr[0]);
-        if (nc[1])
-            dense_closure_warp_kernel<4><<<grids[1], kThreads, 0, p->stream>>>(a, B.chunks + first[1], nc[1], ctr[1]);
-        if (nc[2])
-            dense_closure_warp_kernel<16><<<grids[2], kThreads, 0, p->stream>>>(a, B.chunks + first[2], nc[2], ctr[2]);
-        if (nc[3])
-            dense_closure_kernel<<<grids[3], kThreads, smem, p->stream>>>(a, (u32)cta_wmax, B.chunks + first[3], nc[3],
-                                                                          ctr[3]);
+        for (int sh = 3; sh >= 0; sh--)
+            if (nc[sh])
+                fn[sh]<<<grids[sh], threads[sh], smem[sh], p->stream>>>(a, (u32)nmax[sh], sh == 3 ? B.queue : nullptr,
+                                                                        B.chunks + first[sh], nc[sh], ctr[sh]);
+        if (nc[4])
+            dense_closure_kernel<<<grids[4], kThreads, smem[4], p->stream>>>(a, (u32)(nmax[4] / 32),
+                                                                             B.chunks + first[4], nc[4], ctr[4]);
         for (int sh = 0; sh < kShapes; sh++)
             if (nc[sh]) LAUNCHED();
         if (p->kernel_events) {
@@ -2463,8 +2465,8 @@ bool run_scc_dense(ra_program* p, Scc& s)
             CK(cudaEventRecord(ev[0], p->stream));
         }
         dense_emit_kernel<<<std::min<u64>((rows + kWarps - 1) / kWarps, (u64)kSms * 16), kThreads, 0, p->stream>>>(
-            DenseArgs{B.inst, p->n_inst ? p->dinst_base : nullptr, ninst, rows, B.known, B.delta0, p->bits, sk, scsr,
-                      B.s_local, B.row_new, B.level_total, nullptr, level_cap, B.inst_init, B.counters, B.flags},
+            DenseArgs{B.inst, p->n_inst ? p->dinst_base : nullptr, ninst, rows, B.known, B.known, p->bits, sk, scsr,
+                      B.s_edge, B.row_new, B.level_total, nullptr, level_cap, B.counters, B.flags},
             B.row_off, R.keys + n_stored, R.ids + n_stored, (u64)R.tag << 46, ctr);
         LAUNCHED();
         if (p->kernel_events) {
