@@ -45,6 +45,64 @@ __device__ __forceinline__ u32 lanemask_lt()
     return m;
 }
 
+// position of the (r + 1)-th set bit of w (r < popc(w))
+__device__ __forceinline__ u32 nth_set_bit(u32 w, u32 r)
+{
+    u32 at = 0;
+#pragma unroll
+    for (int h = 16; h; h >>= 1) {
+        const u32 low = __popc(w & ((1u << h) - 1));
+        if (r >= low) {
+            r -= low;
+            w >>= h;
+            at += h;
+        }
+    }
+    return at;
+}
+
+// The set bits of 32 words (lane l's word holds bits 32 l ...) in ascending order:
+// store(t, bit) for the t-th; returns their number.  Called by a whole warp; consecutive
+// lanes store consecutive t.  Few words with many bits: word by word, lane b storing bit b
+// if set; else 32 outputs at a time, a lane finding its word by a search over the lanes'
+// counts and its bit by rank.
+template <typename Store>
+__device__ __forceinline__ u32 emit_words(u32 word, Store store)
+{
+    const int lane = threadIdx.x & 31;
+    const u32 c = __popc(word);
+    u32 incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const u32 total = __shfl_sync(0xffffffffu, incl, 31), before = incl - c;
+    const u32 nz = __ballot_sync(0xffffffffu, word != 0);
+    if ((u32)__popc(nz) <= 4 * ((total + 31) / 32)) {
+        for (u32 m = nz; m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const u32 wj = __shfl_sync(0xffffffffu, word, j), bj = __shfl_sync(0xffffffffu, before, j);
+            if ((wj >> lane) & 1) store(bj + __popc(wj & lanemask_lt()), (u32)j * 32 + lane);
+        }
+        return total;
+    }
+    for (u32 t0 = 0; t0 < total; t0 += 32) {
+        const u32 t = t0 + lane;
+        // first lane j with incl_j > t (every lane joins the shuffles)
+        u32 lo = 0, hi = 31;
+#pragma unroll
+        for (int step = 0; step < 5; step++) {
+            const u32 mid = (lo + hi) >> 1;
+            if (__shfl_sync(0xffffffffu, incl, mid) > t) hi = mid;
+            else lo = mid + 1;
+        }
+        const u32 wj = __shfl_sync(0xffffffffu, word, lo), bj = __shfl_sync(0xffffffffu, before, lo);
+        if (t < total) store(t, lo * 32 + nth_set_bit(wj, t - bj));
+    }
+    return total;
+}
+
 // Inclusive warp scan of u64.
 __device__ __forceinline__ u64 warp_inclusive_scan(u64 v)
 {

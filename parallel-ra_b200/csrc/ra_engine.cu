@@ -1262,7 +1262,11 @@ int launch_iteration(ra_program* p, DevScc& d, cudaGraphConditionalHandle cond, 
         const DevRule& r = d.rules[q];
         Relation& out = p->rels[d.rel_of_slot[r.out_slot]];
         PhaseTimer pt(p, 2);
-        if (r.kind == kJoin)
+        if (r.kind == kJoin && d.bit[r.out_slot].seen && r.longest <= kHeavyRow)
+            join_bitmap_kernel<<<grid_blocks(8), kThreads, 0, p->stream>>>(p->ctl, q, r.in, r.outer_shift, r.csr,
+                                                                           r.inner, r.pj, p->bits,
+                                                                           d.bit[r.out_slot]);
+        else if (r.kind == kJoin)
             join_kernel(r)<<<G, kThreads, 0, p->stream>>>(p->ctl, q, r.in, r.outer_shift, r.csr, r.inner, r.pj,
                                                           p->bits, p->dcand, p->dcand_cap, out.seen, out.seen_cap,
                                                           p->dloser, p->status, p->status_cap, slot++,
@@ -1296,6 +1300,16 @@ int launch_iteration(ra_program* p, DevScc& d, cudaGraphConditionalHandle cond, 
             b.dst_ids = out.ids;
             b.bs = d.bit[r.out_slot];
             b.bits = p->bits;
+            // rows of few words share a tile's look-back, as long as there is a tile for every resident
+            // CTA; wide rows keep a warp each busy.  Measured (1 / 2 / 4 rows per warp): a tree of 2^15
+            // nodes, 1,024 words per row, 8.4 / 8.9 / 9.8 ms; a wave of 96 trees, at most 128 words, 6.2 /
+            // 5.4 / 4.8 ms
+            const u64 brows = d.bit[r.out_slot].n;
+            const u64 bwords = p->n_inst ? p->bmt_total / std::max<u64>(brows, 1) : d.bit[r.out_slot].words;
+            b.rows_per_warp = 1;
+            while (b.rows_per_warp < kBitSelRows && 2 * b.rows_per_warp * bwords <= 512 &&
+                   brows >= (u64)kWarps * 2 * b.rows_per_warp * kSms * 4)
+                b.rows_per_warp *= 2;
             if (p->n_inst) {
                 b.inst_new = p->dinst_new;
                 b.n_inst = p->n_inst;
