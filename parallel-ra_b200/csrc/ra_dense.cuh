@@ -458,11 +458,8 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
 
 // New tuples of each row into the log: row by row (values ascending), within a
 // row by column-0 value ascending; key (z, x), id tag_word | (id_base + position).
-// One warp per row: it takes the row's words 32 at a time, scans their bit
-// counts, and lane t writes output t, t + 32, ... of the group -- consecutive
-// lanes write consecutive rows of the log (coalesced); a lane finds the word
-// holding its output by a binary search over the lanes' inclusive counts and
-// the bit by its rank within the word.
+// One warp per row, 32 words at a time (emit_words): consecutive lanes write consecutive
+// rows of the log (coalesced).
 __global__ void __launch_bounds__(kThreads) dense_emit_kernel(DenseArgs a, const u64* __restrict__ row_off,
                                                               u64* __restrict__ keys_out, u64* __restrict__ ids_out,
                                                               u64 tag_word, u64 id_base)
@@ -477,36 +474,10 @@ __global__ void __launch_bounds__(kThreads) dense_emit_kernel(DenseArgs a, const
         u64 pos = row_off[row];
         for (u32 g = 0; g < W; g += 32) {
             const u32 word = (g + lane < W) ? nrow[g + lane] : 0u;
-            const u32 c = __popc(word);
-            u32 incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const u32 t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const u32 group = __shfl_sync(0xffffffffu, incl, 31);
-            for (u32 t0 = 0; t0 < group; t0 += 32) {
-                const u32 t = t0 + lane;
-                // first lane j with incl_j > t (every lane joins the shuffles)
-                u32 lo = 0, hi = 31;
-#pragma unroll
-                for (int step = 0; step < 5; step++) {
-                    const u32 mid = (lo + hi) >> 1;
-                    const u32 im = __shfl_sync(0xffffffffu, incl, mid);
-                    if (im > t) hi = mid;
-                    else lo = mid + 1;
-                }
-                const u32 wj = __shfl_sync(0xffffffffu, word, lo);
-                const u32 before = __shfl_sync(0xffffffffu, incl - c, lo);
-                if (t < group) {
-                    const u32 bit = __fns(wj, 0, (int)(t - before) + 1);
-                    const u64 z = d.base + (u64)(g + lo) * 32 + bit;
-                    const u64 at = pos + t;
-                    keys_out[at] = (z << a.bits) | row;
-                    ids_out[at] = tag_word | (id_base + at);
-                }
-            }
-            pos += group;
+            pos += emit_words(word, [&](u32 t, u32 bit) {
+                keys_out[pos + t] = ((d.base + (u64)g * 32 + bit) << a.bits) | row;
+                ids_out[pos + t] = tag_word | (id_base + pos + t);
+            });
         }
     }
 }
