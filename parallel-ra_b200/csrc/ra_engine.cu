@@ -19,6 +19,7 @@
 #include "ra_dense.cuh"
 #include "ra_persist.cuh"
 #include "ra_reach.cuh"
+#include "ra_sparse.cuh"
 #include "ra_tail.cuh"
 #include "ra_wide.cuh"
 
@@ -246,6 +247,7 @@ struct ra_program {
     bool use_persist = false;     // RA_PERSIST=1: the persistent SCC kernel instead of CUDA-graph iterations
     bool use_reach = false;       // RA_REACH=1: closure-shaped SCCs by composing reachable sets
     u64 reach_arena_hint = 0;     // arena entries the last reachability evaluation used
+    u64 sp_arena_hint = 0, sp_levels_hint = 0;   // arena and level entries the last sparse row closure used
     bool use_tail = true;         // RA_NO_TAIL=1: no tail kernel in the iteration body
     int tail_ctas = -1;           // CTAs of the tail kernel's cluster (0: none fits; -1: not yet asked)
     bool kernel_events = false;   // RA_KERNEL_EVENTS=1: per-launch events on the claim kernels (no graph)
@@ -2514,6 +2516,170 @@ bool run_scc_dense(ra_program* p, Scc& s)
     return true;
 }
 
+// Is SCC s one rule of the transitive-closure shape R(z, x) :- R_delta(y, x), S_full(y, z)
+// with S fixed, run in emission order one iteration at a time?
+bool closure_shape(ra_program* p, const Scc& s, JoinPlan& jp)
+{
+    if (!s.fixpoint || s.rules.size() != 1 || s.rules[0].kind != kJoin) return false;
+    if (p->id_order != RA_IDS_EMISSION || p->batch_size != 1 || p->cp_every) return false;
+    const Rule& ru = s.rules[0];
+    jp = make_join_plan(p, ru);
+    if (jp.outer_rel != ru.out || jp.outer_ver != RA_DELTA || jp.inner_ver != RA_FULL || jp.inner_rel == ru.out)
+        return false;
+    const Relation& R = p->rels[ru.out];
+    const Relation& S = p->rels[jp.inner_rel];
+    if (R.arity != 2 || S.arity != 2 || R.jcc != 1) return false;
+    const Projection& pj = jp.pj;
+    if (pj.n != 2 || pj.side[0] != 1 || pj.col[0] != 1 || pj.side[1] != 0 || pj.col[1] != 1) return false;
+    return std::find(s.rels.begin(), s.rels.end(), jp.inner_rel) == s.rels.end() || S.delta_n == 0;
+}
+
+// Device buffers of one sparse row closure, freed on every exit.
+struct SparseBufs {
+    ra_program* p;
+    u64 *first = nullptr, *adj = nullptr, *tile_at = nullptr, *tile_lv = nullptr, *ctr = nullptr, *base = nullptr;
+    u32 *target = nullptr, *queue = nullptr, *arena = nullptr, *levels = nullptr, *pos = nullptr, *tile_nlv = nullptr;
+    u32 *block_lv = nullptr, *flags = nullptr, *big_queue = nullptr;
+    u16 *warp_lv = nullptr, *big_table = nullptr;
+    explicit SparseBufs(ra_program* pp) : p(pp) {}
+    ~SparseBufs()
+    {
+        for (u64** q : {&first, &adj, &tile_at, &tile_lv, &ctr, &base}) dev_free(p, q);
+        for (u32** q : {&target, &queue, &arena, &levels, &pos, &tile_nlv, &block_lv, &flags, &big_queue})
+            dev_free(p, q);
+        dev_free(p, &warp_lv);
+        dev_free(p, &big_table);
+    }
+};
+
+// Runs SCC s with the sparse row closure (ra_sparse.cuh) when its one rule has the
+// transitive-closure shape, the values are too many for the dense evaluator's bit matrices and
+// every row's search stays small; returns false (nothing done) otherwise: the loop runs it.
+// Leaves the relations, the log with its ids and the history as the loop would.  A memory
+// cap, per-launch events, instances and the opt-in evaluators keep the loop, and so does a
+// dense budget of 0, which switches off every evaluator of this shape.
+bool run_scc_sparse(ra_program* p, Scc& s)
+{
+    JoinPlan jp;
+    if (!closure_shape(p, s, jp)) return false;
+    if (p->n_inst || p->use_persist || p->kernel_events || p->alloc_cap || p->tune.dense_max_bytes <= 0) return false;
+    Relation& R = p->rels[s.rules[0].out];
+    Relation& S = p->rels[jp.inner_rel];
+    const u64 n = p->max_value + 1;
+    if (R.full_n != 0 || R.delta_n == 0) return false;
+    if (n <= kDenseMaxN || p->bits + kSpShift > 31) return false;
+    const u64 *sk, *sv;
+    u64 sn;
+    version_rows(p, S, RA_FULL, &sk, &sv, &sn);
+    if (sn == 0 || n > 16 * sn + (1u << 18)) return false;   // per-value arrays would dwarf the input
+    const u64* scsr = version_csr(p, S, RA_FULL);
+    const u64 n_stored = R.delta_n;
+    SparseBufs B(p);
+    SparseArgs a{};
+    a.n = n;
+    a.bits = p->bits;
+    a.tiles = (u32)((n + kSpRows - 1) >> kSpShift);
+    a.blocks = (a.tiles + (1u << kSpBlockShift) - 1) >> kSpBlockShift;
+    a.delta = R.keys;
+    a.n_delta = n_stored;
+    a.arena_cap = std::max<u64>(p->sp_arena_hint, 24 * sn + (1u << 20));
+    a.levels_cap = std::max<u64>(p->sp_levels_hint, 48ull * a.tiles + (1u << 16));
+    static int occ = 0;
+    if (!occ) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sparse_search_kernel, kSpWarps * 32, 0));
+    const int grid = (int)std::min<u64>((u64)kSms * std::max(occ, 1), (a.tiles + kSpWarps - 1) / kSpWarps);
+    a.big = std::min<u32>(kSpBig, 16 + a.tiles / 64);
+    std::vector<u64> total(kSpLevels), hc(4);
+    u32 fl = 0;
+    try {
+        dev_alloc(p, &B.first, a.tiles + 1);
+        dev_alloc(p, &B.adj, n);
+        dev_alloc(p, &B.target, sn);
+        dev_alloc(p, &B.queue, (u64)grid * kSpWarps * kSpQueue);
+        dev_alloc(p, &B.warp_lv, (u64)grid * kSpWarps * kSpLevels);
+        dev_alloc(p, &B.big_queue, (u64)a.big * kSpBigQueue);
+        dev_alloc(p, &B.big_table, (u64)a.big * kSpBigSlots);
+        dev_alloc(p, &B.tile_at, a.tiles);
+        dev_alloc(p, &B.tile_lv, a.tiles);
+        dev_alloc(p, &B.tile_nlv, a.tiles);
+        dev_alloc(p, &B.block_lv, (u64)a.blocks * kSpLevels);
+        dev_alloc(p, &B.ctr, 5 + kSpLevels);
+        dev_alloc(p, &B.base, kSpLevels);
+        dev_alloc(p, &B.flags, 1);
+        a.first = B.first;
+        a.adj = B.adj;
+        a.target = B.target;
+        a.queue = B.queue;
+        a.warp_lv = B.warp_lv;
+        a.big_queue = B.big_queue;
+        a.big_table = B.big_table;
+        a.tile_at = B.tile_at;
+        a.tile_lv = B.tile_lv;
+        a.tile_nlv = B.tile_nlv;
+        a.block_lv = B.block_lv;
+        a.ctr = B.ctr;
+        a.level_total = B.ctr + 5;
+        a.flags = B.flags;
+        CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
+        sparse_adj_kernel<<<grid_for(std::max(n, sn)), kThreads, 0, p->stream>>>(a, scsr, sk, sn);
+        LAUNCHED();
+        sparse_bounds_kernel<<<grid_for(n_stored + 1), kThreads, 0, p->stream>>>(a);
+        LAUNCHED();
+        for (int round = 0;; round++) {
+            dev_free(p, &B.arena);
+            dev_free(p, &B.levels);
+            dev_free(p, &B.pos);
+            dev_alloc(p, &B.arena, a.arena_cap);
+            dev_alloc(p, &B.levels, a.levels_cap);
+            dev_alloc(p, &B.pos, a.levels_cap);
+            a.arena = B.arena;
+            a.levels = B.levels;
+            CK(cudaMemsetAsync(B.block_lv, 0, (u64)a.blocks * kSpLevels * 4, p->stream));
+            CK(cudaMemsetAsync(B.ctr, 0, (5 + kSpLevels) * 8, p->stream));
+            sparse_search_kernel<<<grid, kSpWarps * 32, 0, p->stream>>>(a);
+            LAUNCHED();
+            sparse_scan_kernel<<<kSpLevels / kWarps, kThreads, 0, p->stream>>>(a);
+            LAUNCHED();
+            CK(cudaMemcpyAsync(&fl, B.flags, 4, cudaMemcpyDeviceToHost, p->stream));
+            CK(cudaMemcpyAsync(hc.data(), B.ctr, 4 * 8, cudaMemcpyDeviceToHost, p->stream));
+            CK(cudaMemcpyAsync(total.data(), a.level_total, kSpLevels * 8, cudaMemcpyDeviceToHost, p->stream));
+            CK(cudaStreamSynchronize(p->stream));
+            if (fl & ~kSpArena) return false;
+            if (!(fl & kSpArena)) break;
+            if (round) return false;
+            a.arena_cap = std::max(a.arena_cap, hc[1]);   // the whole search's needs are known
+            a.levels_cap = std::max(a.levels_cap, hc[2]);
+            CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
+        }
+        p->sp_arena_hint = hc[1] + hc[1] / 8;
+        p->sp_levels_hint = hc[2] + hc[2] / 8;
+        ensure_log(p, R, n_stored + hc[1]);
+    } catch (const ra_error& e) {
+        if (e.status != RA_E_OOM) throw;
+        p->err.clear();   // no room for the scratch
+        cudaGetLastError();
+        return false;
+    }
+    u64 L = 0, sum = 0;
+    std::vector<u64> base(kSpLevels, 0);
+    for (; L < kSpLevels && total[L]; L++) {
+        base[L] = sum;
+        sum += total[L];
+    }
+    if (sum) {
+        const u64 id0 = ((u64)R.tag << 46) | intern_counter(p, R.tag);
+        CK(cudaMemcpyAsync(B.base, base.data(), L * 8, cudaMemcpyHostToDevice, p->stream));
+        sparse_offsets_kernel<<<a.blocks, kThreads, 0, p->stream>>>(a, B.pos);
+        LAUNCHED();
+        sparse_place_kernel<<<(int)std::min<u64>((a.tiles + kWarps - 1) / kWarps, kSms * 8), kThreads, 0, p->stream>>>(
+            a, B.pos, B.base, R.keys + n_stored, R.ids + n_stored, id0);
+        LAUNCHED();
+        CK(cudaStreamSynchronize(p->stream));   // the scratch goes when this returns
+    }
+    p->stats.join_candidates += hc[3];
+    finish_closure_scc(p, s, s.rules[0].out, R, n_stored, sum, total, L, L + 1);
+    return true;
+}
+
 // Device buffers of one reachability evaluation, freed on every exit.
 struct ReachBufs {
     ra_program* p;
@@ -2859,7 +3025,7 @@ void run_scc(ra_program* p, Scc& s)
         for (size_t i = 0; i < s.rels.size(); i++)
             if (s.init[i]) full_to_delta(p, p->rels[s.rels[i]]);
     }
-    if (run_scc_dense(p, s) || run_scc_reach(p, s)) {
+    if (run_scc_dense(p, s) || run_scc_reach(p, s) || run_scc_sparse(p, s)) {
         p->pending_merge = s.rels;
         return;
     }

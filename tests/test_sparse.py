@@ -1,0 +1,124 @@
+"""The sparse row closure (a transitive-closure-shaped SCC over more than 65,536 values whose
+rows stay small, one warp per 16 rows) leaves what the iteration loop leaves: history,
+rows and ids; what it cannot hold goes to the loop."""
+import numpy as np
+import pytest
+
+import oracle as O
+import parallel_ra_b200 as P
+
+pytestmark = pytest.mark.gpu
+
+N = 70_001   # above the dense evaluator's range, not a multiple of a tile
+
+
+def er(n, m, seed):
+    return P.datagen.erdos_renyi(n, m, seed)
+
+
+def path(length, start, step=1):
+    v = np.arange(start, start + step * length + 1, step, dtype=np.uint64)
+    return np.stack([v[:-1], v[1:]], axis=1)
+
+
+def comb():
+    """Node 3 reaches 100, 31, 32, 33 and 1 direct successors at different levels."""
+    edges, nxt, at = [], 20, 3
+    for width in (100, 31, 32, 33, 1):
+        kids = np.arange(nxt, nxt + width)
+        edges += [(at, k) for k in kids] + [(kids[0], kids[-1]), (kids[-1], at)]   # duplicates and a cycle
+        at, nxt = kids[width // 2], nxt + width
+    return np.array(edges, dtype=np.uint64)
+
+
+def with_top(edges):
+    return np.concatenate([edges, np.array([[N - 1, N - 2]], dtype=np.uint64)])
+
+
+# (edges, does the sparse closure take them)
+CASES = {
+    "sparse": (lambda: er(N, N // 2, 1), True),
+    "er_0.95": (lambda: er(N, round(0.95 * N), 2), True),
+    "path": (lambda: with_top(path(500, 5)), True),                       # 16 rows of 500 tuples in a tile
+    "longer_path": (lambda: with_top(path(1000, 5)), True),               # 16,000: the large queues
+    "a_thousand_levels": (lambda: with_top(path(1000, 5, 16)), True),     # a row per tile, levels of width 1
+    "too_many_levels": (lambda: with_top(path(1100, 5, 16)), False),
+    "comb": (lambda: with_top(comb()), True),
+    "self_loops_duplicates": (lambda: with_top(np.array([[0, 0], [0, 1], [0, 1], [1, 0], [16, 15], [15, 16]],
+                                                        dtype=np.uint64)), True),
+    "initial_rows_fill_a_tile": (lambda: with_top(np.stack([np.full(32768, 7), np.arange(1000, 33768)], axis=1)
+                                                  .astype(np.uint64)), True),
+    "initial_rows_outgrow_a_tile": (lambda: with_top(np.stack([np.full(32769, 7), np.arange(1000, 33769)], axis=1)
+                                                     .astype(np.uint64)), False),
+    "a_tile_outgrows_its_queue": (lambda: with_top(np.concatenate([
+        path(20, 16), np.stack([np.full(500, 36), np.arange(1000, 1500)], axis=1).astype(np.uint64)])), True),
+    "a_tile_outgrows_a_large_queue": (lambda: with_top(np.concatenate([
+        path(20, 16), np.stack([np.full(2100, 36), np.arange(1000, 3100)], axis=1).astype(np.uint64)])), False),
+    "cycle_of_a_thousand": (lambda: with_top(np.concatenate([path(999, 100), np.array([[1099, 100]], dtype=np.uint64)])),
+                              True),
+}
+
+
+def run(rows, loop=False):
+    p = P.Program(0)
+    if loop:
+        p.set_tuning(dense_max_bytes=0)
+    rels = P.programs.build_tc(p, rows)
+    p.execute(1)
+    return p, rels
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_sparse_closure_leaves_what_the_loop_leaves(case):
+    make, taken = CASES[case]
+    rows = P.datagen.with_row_ids(make())
+    a, ra = run(rows)
+    b, rb = run(rows, loop=True)
+    assert (a.stats().dedup_launches == 1) == taken   # the copy rule's launch, and the loop's joins otherwise
+    assert b.stats().dedup_launches > 1
+    assert a.history() == b.history()
+    assert a.stats().join_candidates == b.stats().join_candidates
+    for name in ra:
+        assert a.counts(ra[name]) == b.counts(rb[name])
+        assert np.array_equal(a.dump_full(ra[name]), b.dump_full(rb[name])), name   # ids included
+    o = O.OracleProgram()
+    ro = P.programs.build_tc(o, rows)
+    o.execute(1)
+    assert a.history() == o.history()
+    assert np.array_equal(a.dump_full(ra["T"])[:, :2], o.dump_full(ro["T"])[:, :2])
+
+
+def test_an_initial_delta_not_grouped_by_source_goes_to_the_loop():
+    rows = P.datagen.with_row_ids(er(N, N // 2, 5))
+    got = []
+    for loop in (False, True):
+        p = P.Program(0)
+        if loop:
+            p.set_tuning(dense_max_bytes=0)
+        T = p.relation(1, 2, 257, "T")
+        G = p.relation(1, 2, 256, "G")
+        p.load_rows(T, np.empty((0, 3), dtype=np.uint64))
+        p.load_rows(G, rows)
+        copy, join = p.scc(False, 2), p.scc(True, 1)
+        for s in (copy, join):
+            p.add_relation(s, G, False)
+            p.add_relation(s, T, True)
+        p.copy(copy, T, G, P.engine.FULL, [0, 1])            # T(src, dst): column 1 in no order
+        p.join(join, T, T, P.engine.DELTA, G, P.engine.FULL, [3, 1])
+        p.depend(copy, join)
+        p.execute(1)
+        got.append((p.history(), p.dump_full(T), p.stats().dedup_launches))
+    assert got[0][0] == got[1][0] and got[0][2] > 1
+    assert np.array_equal(got[0][1], got[1][1])
+
+
+def test_runs_repeat_and_other_inputs_follow():
+    p = P.Program(0)
+    rels = P.programs.build_tc(p, np.empty((0, 3), dtype=np.uint64))
+    for n, m, seed in ((N, 30_000, 1), (3 * N, 2 * N, 2), (N, 60_000, 3), (500, 600, 4), (N, 60_000, 3)):
+        rows = P.datagen.with_row_ids(er(n, m, seed))
+        p.load_rows(rels["G"], rows)
+        p.execute(1)
+        q, rq = run(rows, loop=True)
+        assert p.history() == q.history()
+        assert np.array_equal(p.dump_full(rels["T"])[:, :2], q.dump_full(rq["T"])[:, :2])
