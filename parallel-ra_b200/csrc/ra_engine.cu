@@ -30,7 +30,10 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <condition_variable>
 #include <functional>
+#include <mutex>
+#include <thread>
 #include <fstream>
 #include <string>
 #include <sys/stat.h>
@@ -343,6 +346,134 @@ u64 read_scalar(ra_program* p, const u64* dptr)
     CK(cudaMemcpyAsync(p->hscalar, dptr, 8, cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     return p->hscalar[0];
+}
+
+// Pinned staging of large reads to the host, shared by the process's programs: 12 MB, made
+// by the first such read (pinning costs milliseconds), freed with the last program.  One
+// read uses it at a time; another one meanwhile takes the plain copy.
+constexpr u64 kRingChunk = 2u << 20;
+constexpr int kRingChunks = 6;
+constexpr int kRingThreads = 4;
+constexpr u64 kRingBytes = 12u << 20;   // reads below are plain copies
+
+struct HostRing {
+    std::mutex busy;          // held while a read uses (or frees) the buffer
+    std::mutex count_mu;
+    int programs = 0;
+    char* buf = nullptr;
+    void add()
+    {
+        std::lock_guard<std::mutex> lk(count_mu);
+        programs++;
+    }
+    void remove()
+    {
+        std::lock_guard<std::mutex> lk(count_mu);
+        if (--programs) return;
+        std::lock_guard<std::mutex> use(busy);
+        if (buf) cudaFreeHost(buf);
+        buf = nullptr;
+    }
+};
+HostRing g_ring;
+
+// Device bytes to pageable host memory, complete on return.  A plain copy is bound by one
+// thread of the driver that moves staged bytes into the caller's pages, faults of fresh
+// pages included.  Large reads land chunk by chunk in a pinned ring, and four threads move
+// the chunks on.  Measured (16-core host): 45 MB of fresh rows 10.7 -> 3.4 ms, of touched
+// ones 2.8 -> 2.0; 100 MB fresh 22.5 -> 7.6; 16 MB 1.45 -> 1.0; 8 MB 0.72 -> 0.92, so these stay
+// plain.  Chunks of 512 KB and eight threads: 30 MB touched 6.3 ms against 1.4 (the threads
+// meet in one huge page, and at the lock).
+void rows_to_host(ra_program* p, void* dst, const void* src, u64 bytes)
+{
+    std::unique_lock<std::mutex> use(g_ring.busy, std::defer_lock);
+    bool ring = bytes >= kRingBytes && std::thread::hardware_concurrency() >= 2 * kRingThreads && use.try_lock();
+    if (ring && !g_ring.buf && cudaHostAlloc((void**)&g_ring.buf, kRingChunk * kRingChunks, cudaHostAllocPortable) !=
+                                   cudaSuccess) {
+        cudaGetLastError();
+        g_ring.buf = nullptr;
+        ring = false;
+    }
+    struct Events {
+        cudaEvent_t e[kRingChunks] = {};
+        ~Events()
+        {
+            for (cudaEvent_t v : e)
+                if (v) cudaEventDestroy(v);
+        }
+    } ev;
+    for (int i = 0; i < kRingChunks && ring; i++) CK(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming));
+    if (!ring) {
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, p->stream));
+        CK(cudaStreamSynchronize(p->stream));
+        return;
+    }
+    char* const buf = g_ring.buf;
+    const u64 chunks = (bytes + kRingChunk - 1) / kRingChunk;
+    auto move_on = [&](u64 i) {
+        const u64 at = i * kRingChunk;
+        std::memcpy((char*)dst + at, buf + (i % kRingChunks) * kRingChunk, std::min(kRingChunk, bytes - at));
+    };
+    std::vector<char> moved(chunks, 0);
+    std::mutex mu;
+    std::condition_variable more, room;   // a chunk landed (or the read ended); a chunk was moved on
+    u64 ready = 0, taken = 0;             // chunks landed, chunks a thread has taken
+    bool end = false;
+    auto work = [&]() {
+        std::unique_lock<std::mutex> lk(mu);
+        for (;;) {
+            more.wait(lk, [&] { return end || taken < ready; });
+            if (taken >= ready) return;
+            const u64 i = taken++;
+            lk.unlock();
+            move_on(i);
+            lk.lock();
+            moved[i] = 1;
+            room.notify_one();
+        }
+    };
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(kRingThreads);
+        for (int t = 0; t < kRingThreads; t++) pool.emplace_back(work);
+    } catch (...) {   // as many threads as could be had; none: this one moves the chunks
+    }
+    cudaError_t err = cudaSuccess;
+    u64 issued = 0;
+    for (u64 landed = 0; landed < chunks && err == cudaSuccess; landed++) {
+        while (issued < chunks && issued < landed + kRingChunks && err == cudaSuccess) {
+            if (issued >= (u64)kRingChunks && !pool.empty()) {   // its slot's last chunk must have left
+                std::unique_lock<std::mutex> lk(mu);
+                const u64 old = issued - kRingChunks;
+                if (issued > landed && !moved[old]) break;   // other chunks are in flight: see to those
+                room.wait(lk, [&] { return moved[old] != 0; });
+            }
+            const u64 at = issued * kRingChunk, slot = issued % kRingChunks;
+            err = cudaMemcpyAsync(buf + slot * kRingChunk, (const char*)src + at, std::min(kRingChunk, bytes - at),
+                                  cudaMemcpyDeviceToHost, p->stream);
+            if (err == cudaSuccess) err = cudaEventRecord(ev.e[slot], p->stream);
+            issued++;
+        }
+        if (err == cudaSuccess) err = cudaEventSynchronize(ev.e[landed % kRingChunks]);
+        if (err != cudaSuccess) break;
+        if (pool.empty()) {
+            move_on(landed);
+            continue;
+        }
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            ready = landed + 1;
+        }
+        more.notify_one();
+    }
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        end = true;
+    }
+    more.notify_all();
+    for (std::thread& t : pool) t.join();
+    if (err != cudaSuccess) cudaStreamSynchronize(p->stream);   // no copy still writes the ring
+    ck(p, err, "rows to host");
 }
 
 // ---------------------------------------------------------------------------
@@ -3344,6 +3475,7 @@ int ra_program_create(int device, ra_program** out)
         delete p;
         return st;
     }
+    g_ring.add();
     *out = p;
     return RA_OK;
 }
@@ -3409,6 +3541,7 @@ int ra_program_destroy(ra_program* p)
     if (p->ev1) cudaEventDestroy(p->ev1);
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
+    g_ring.remove();
     return RA_OK;
 }
 
@@ -3917,8 +4050,7 @@ int ra_relation_dump_full(ra_program* p, int rel, uint64_t* host_rows, uint64_t 
         if (p->wide) {   // rows already in trie order
             const u64 m = std::min<u64>(r.full_n, cap_rows);
             if (rows_out) *rows_out = m;
-            if (m && host_rows)
-                CK(cudaMemcpyAsync(host_rows, r.wfull, m * (r.arity + 1) * 8, cudaMemcpyDeviceToHost, p->stream));
+            if (m && host_rows) rows_to_host(p, host_rows, r.wfull, m * (r.arity + 1) * 8);
             CK(cudaStreamSynchronize(p->stream));
             return;
         }
@@ -3932,9 +4064,12 @@ int ra_relation_dump_full(ra_program* p, int rel, uint64_t* host_rows, uint64_t 
         dev_alloc(p, &rows, m * (r.arity + 1));
         rows_unpack<<<grid_for(m), kThreads, 0, p->stream>>>(k, v, m, (int)r.arity, p->bits, rows);
         LAUNCHED();
-        CK(cudaMemcpyAsync(host_rows, rows, m * (r.arity + 1) * 8, cudaMemcpyDeviceToHost, p->stream));
-        dev_free(p, &rows);
-        CK(cudaStreamSynchronize(p->stream));
+        struct Free {
+            ra_program* p;
+            u64** q;
+            ~Free() { dev_free(p, q); }
+        } free_rows{p, &rows};
+        rows_to_host(p, host_rows, rows, m * (r.arity + 1) * 8);
     });
 }
 
