@@ -88,22 +88,25 @@ void wide_scan_async(ra_program* p, const T* in, u64 n, u64* out, u64* total_dev
     CK(cudaMemcpyAsync(total_dev, p->dscalar, 8, cudaMemcpyDeviceToDevice, p->stream));
 }
 
+// The block sorts' dynamic shared memory (rows of a tile), above the default limit.
+void wide_allow_smem(ra_program* p)
+{
+    CK(cudaFuncSetAttribute(wide_tile_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem));
+    CK(cudaFuncSetAttribute(wide_newt_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem));
+}
+
 // Indices 0..n-1 of `rows` sorted by (first ncmp columns, index); the result is
 // one of the two index scratch slots.
 const u64* wide_sort(ra_program* p, const u64* rows, int W, int ncmp, u64 n)
 {
     u64* a = wide_scratch(p, kWsIdxA, n);
     u64* b = wide_scratch(p, kWsIdxB, n);
-    if (n <= 64) {
-        wide_tile_sort_kernel<64><<<1, kThreads, 0, p->stream>>>(rows, W, ncmp, n, a);
-    } else if (n <= 256) {
-        wide_tile_sort_kernel<256><<<1, kThreads, 0, p->stream>>>(rows, W, ncmp, n, a);
-    } else {
-        const u64 tiles = (n + kWideSortTile - 1) / kWideSortTile;
-        wide_tile_sort_kernel<kWideSortTile><<<(unsigned)tiles, kThreads, 0, p->stream>>>(rows, W, ncmp, n, a);
-    }
+    const u64 tile = wide_tile_rows(W);
+    wide_allow_smem(p);
+    wide_tile_sort_kernel<<<(unsigned)((n + tile - 1) / tile), kWideBlockSort, std::min(n, tile) * W * 8, p->stream>>>(
+        rows, W, ncmp, n, (u32)tile, a);
     LAUNCHED();
-    for (u64 L = kWideSortTile; L < n; L *= 2) {
+    for (u64 L = tile; L < n; L *= 2) {
         wide_merge_pass_kernel<<<wide_grid(n), kThreads, 0, p->stream>>>(rows, W, ncmp, n, L, a, b);
         LAUNCHED();
         std::swap(a, b);
@@ -267,6 +270,22 @@ struct WideOut {
     u64 winners = 0;
     std::vector<u64> seg_wins;      // winners before each segment, then the total
 };
+
+// Head flags of a large candidate buffer (wide_heads_*_kernel).
+template <typename T>
+void wide_heads(ra_program* p, Relation& R, u64 n, int cw)
+{
+    const u64 slots = 2 * n, per = 8 / sizeof(T);
+    u64* hash = wide_scratch(p, kWsIdxA, n);
+    T* at = (T*)wide_scratch(p, kWsIdxB, (n + per - 1) / per);
+    T* slot = (T*)wide_scratch(p, kWsRows, (slots + per - 1) / per);
+    wide_heads_hash_kernel<T><<<wide_grid(slots), kThreads, 0, p->stream>>>(R.wcand, cw, n, hash, slot, slots);
+    LAUNCHED();
+    wide_heads_group_kernel<T><<<wide_grid(n), kThreads, 0, p->stream>>>(R.wcand, cw, n, hash, slot, slots, at);
+    LAUNCHED();
+    wide_heads_flag_kernel<T><<<wide_grid(n), kThreads, 0, p->stream>>>(n, slot, at, R.wflag);
+    LAUNCHED();
+}
 
 // Inputs of one rule in the running iteration.
 struct WideRuleRun {
@@ -476,9 +495,8 @@ void wide_iteration(ra_program* p, Scc& s)
                 if (hb.n == kWideJobs) flush_heads();
                 continue;
             }
-            const u64* idx = wide_sort(p, R.wcand, wo.cw, wo.cw, wo.n);
-            wide_head_flags_kernel<<<wide_grid(wo.n), kThreads, 0, p->stream>>>(R.wcand, wo.cw, idx, wo.n, R.wflag);
-            LAUNCHED();
+            if (2 * wo.n < 0xffffffffull) wide_heads<u32>(p, R, wo.n, wo.cw);
+            else wide_heads<u64>(p, R, wo.n, wo.cw);
         }
         flush_heads();
         // membership of the heads in full and delta, one thread per candidate of every relation
@@ -565,19 +583,20 @@ void wide_iteration(ra_program* p, Scc& s)
     // 5. newt rows, sorted into trie order
     {
         PhaseTimer pt(p, 4);
-        u64 small_rows = 0;   // scratch for the batched relations' unsorted rows
-        for (WideOut& wo : outs)
-            if (wo.winners && wo.winners <= kWideBlockSort) small_rows += wo.winners * (p->rels[wo.rel].arity + 1);
-        u64* srows = small_rows ? wide_scratch(p, kWsRows, small_rows) : nullptr;
-        u64 srow_at = 0;
+        auto fits = [&](const WideOut& wo) {   // one block's rows in shared memory
+            return wo.winners <= kWideBlockSort && wo.winners * (p->rels[wo.rel].arity + 1) * 8 <= kWideSmem;
+        };
+        u64 smem = 0;
         WideNewtBatch nb{};
         int nseg_at = 0;
         auto flush_newt = [&]() {
             if (!nb.n) return;
-            wide_newt_batch_kernel<<<nb.n, kWideWideBlock, 0, p->stream>>>(nb);
+            wide_allow_smem(p);
+            wide_newt_batch_kernel<<<nb.n, kWideWideBlock, smem, p->stream>>>(nb);
             LAUNCHED();
             nb.n = 0;
             nseg_at = 0;
+            smem = 0;
         };
         for (WideOut& wo : outs) {
             Relation& R = p->rels[wo.rel];
@@ -585,23 +604,20 @@ void wide_iteration(ra_program* p, Scc& s)
             const int W = (int)R.arity + 1;
             const int nseg = (int)wo.rules.size();
             p->stats.new_tuples += wo.winners;
-            if (wo.winners <= kWideBlockSort) {
+            if (fits(wo)) {
                 if (nseg_at + nseg > 2 * kWideJobs) flush_newt();
                 WideNewtJob& j = nb.job[nb.n++];
-                j = WideNewtJob{R.wcand, R.wflag, R.wpos, srows + srow_at, R.wnewt, wo.n, wo.winners, wo.cw, W,
-                                nseg_at, nseg};
+                j = WideNewtJob{R.wcand, R.wflag, R.wpos, R.wnewt, wo.n, wo.winners, wo.cw, W, nseg_at, nseg};
+                smem = std::max<u64>(smem, wo.winners * (u64)W * 8);
                 for (int k = 0; k < nseg; k++) {
                     nb.seg_start[nseg_at + k] = wo.seg_start[k];
                     nb.win_base[nseg_at + k] = wo.seg_wins[k];
                     nb.id_base[nseg_at + k] = id_base[wo.rules[k]];
                 }
                 nseg_at += nseg;
-                srow_at += wo.winners * (u64)W;
                 if (nb.n == kWideJobs) flush_newt();
                 continue;
             }
-            flush_newt();   // the large path reuses the row scratch
-            srow_at = 0;
             WideSegs sg{};
             sg.n = nseg;
             for (int k = 0; k < sg.n; k++) {
@@ -610,8 +626,7 @@ void wide_iteration(ra_program* p, Scc& s)
                 sg.id_base[k] = id_base[wo.rules[k]];
             }
             sg.start[sg.n] = wo.n;
-            u64* rows = wide_scratch(p, kWsRows, std::max<u64>(wo.winners * (u64)W, small_rows));
-            srows = rows;
+            u64* rows = wide_scratch(p, kWsRows, wo.winners * (u64)W);
             wide_newt_kernel<<<wide_grid(wo.n), kThreads, 0, p->stream>>>(R.wcand, wo.cw, wo.n, R.wflag, R.wpos, sg,
                                                                            W, rows);
             LAUNCHED();

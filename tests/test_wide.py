@@ -289,3 +289,34 @@ def test_wide_restart_from_own_dump(tmp_path):
     assert [sid for sid, _ in q.history()] == [1]
     p.close()
     q.close()
+
+
+# rows per sort at the edges of a warp, of the shuffle / shared-memory stages, of a block and of
+# several tiles; widths that change the tile; leading columns that agree, ranges that fill the
+# packed key
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,width,kind", [(1, 3, "wide"), (31, 5, "agree"), (33, 24, "agree"), (64, 12, "wide"),
+                                          (65, 41, "agree"), (255, 9, "agree"), (257, 62, "wide"), (512, 21, "agree"),
+                                          (1023, 20, "wide"), (1024, 21, "agree"), (1025, 41, "agree"),
+                                          (3000, 10, "agree"), (5000, 62, "wide")])
+def test_sorted_loads_and_copies(n, width, kind):
+    rng = np.random.default_rng(n + width)
+    rows = rng.integers(0, 2**63, size=(n, width + 1), dtype=np.uint64)
+    if kind == "agree":   # most columns agree, the others differ by little
+        rows[:, :-1] = rows[0, :-1]
+        for c in (width // 2, width - 1):
+            rows[:, c] += rng.integers(0, 40, size=n, dtype=np.uint64)
+    rows[n // 2] = rows[0]   # an exact duplicate
+    got = []
+    for p in (P.Program(0), O.OracleProgram()):
+        a = p.relation(1, width, 300, "A")
+        b = p.relation(1, width, 301, "B")
+        p.load_rows(a, rows)
+        p.load_rows(b, np.empty((0, width + 1), dtype=np.uint64))
+        s = p.scc(False, 1)
+        p.add_relation(s, a, False)
+        p.add_relation(s, b, True)
+        p.copy(s, b, a, 1, list(range(width - 1, -1, -1)))   # columns reversed: new rows to sort
+        p.execute(1)
+        got.append([p.dump_full(a), p.dump_full(b)])
+    assert all(np.array_equal(x, y) for x, y in zip(*got))
