@@ -164,6 +164,9 @@ struct ra_program {
     u64 max_value = 0;            // largest data value loaded (sets `bits`)
     bool packed = false;          // loaded relations packed with `bits` (cleared by a new load)
     bool wide = false;            // this run keeps tuples as rows of u64 columns (ra_wide.cu)
+    cudaEvent_t wide_ev = nullptr;   // what the host waits for in a wide iteration
+    u64* hwide = nullptr;         // page-locked counts of a wide iteration (wide_host_words)
+    u64 hwide_cap = 0;
     u64* wbuf[12] = {};           // scratch of the wide path
     u64 wbuf_cap[12] = {};
     bool executed = false;
@@ -3535,6 +3538,8 @@ int ra_program_destroy(ra_program* p)
         cudaEventDestroy(e.second);
     }
     if (p->stream) cudaStreamSynchronize(p->stream);
+    if (p->hwide) cudaFreeHost(p->hwide);
+    if (p->wide_ev) cudaEventDestroy(p->wide_ev);
     if (p->hscalar) cudaFreeHost(p->hscalar);
     if (p->hctl) cudaFreeHost(p->hctl);
     if (p->ev0) cudaEventDestroy(p->ev0);

@@ -30,7 +30,7 @@
 // (Included inside the engine's anonymous namespace.)
 
 // Scratch slots of the wide path (grow-only, contents not kept across calls).
-enum WideSlot { kWsIdxA, kWsIdxB, kWsRows, kWsLo, kWsCnt, kWsOff, kWsPos, kWsFlag, kWsSmall, kWsTot, kWsCount };
+enum WideSlot { kWsIdxA, kWsIdxB, kWsRows, kWsLo, kWsCnt, kWsOff, kWsPos, kWsFlag, kWsPlace, kWsCount };
 static_assert(kWsCount <= 12, "wide scratch slots");
 
 u64* wide_scratch(ra_program* p, int slot, u64 n)
@@ -74,18 +74,35 @@ void wide_reserve32(ra_program* p, u32** buf, u64* cap, u64 n)
 
 int wide_grid(u64 n) { return grid_for(std::max<u64>(n, 1)); }
 
-// Exclusive scan of n values into out, the total into *total_dev, with no host
-// round trip (one block for small inputs).
+// Page-locked words that kernels write an iteration's counts to, for the host to read after
+// its next synchronisation (a copy back costs two extra operations per round trip).
+u64* wide_host_words(ra_program* p, u64 n)
+{
+    if (n > p->hwide_cap) {
+        if (p->hwide) {
+            CK(cudaStreamSynchronize(p->stream));   // nothing still writes the old words
+            cudaFreeHost(p->hwide);
+        }
+        p->hwide = nullptr;
+        p->hwide_cap = 0;
+        CK(cudaMallocHost(&p->hwide, n * 8));
+        p->hwide_cap = n;
+    }
+    return p->hwide;
+}
+
+// Exclusive scan of n values into out, the total into *total (device or page-locked), with
+// no host round trip (one block for small inputs).
 template <typename T>
-void wide_scan_async(ra_program* p, const T* in, u64 n, u64* out, u64* total_dev)
+void wide_scan_async(ra_program* p, const T* in, u64 n, u64* out, u64* total)
 {
     if (n <= (u64)kThreads * kWideScanPer) {
-        wide_scan_small_kernel<T><<<1, kThreads, 0, p->stream>>>(in, n, out, total_dev);
+        wide_scan_small_kernel<T><<<1, kThreads, 0, p->stream>>>(in, n, out, total);
         LAUNCHED();
         return;
     }
     scan_exclusive<T>(p, in, n, out, false);
-    CK(cudaMemcpyAsync(total_dev, p->dscalar, 8, cudaMemcpyDeviceToDevice, p->stream));
+    CK(cudaMemcpyAsync(total, p->dscalar, 8, cudaMemcpyDefault, p->stream));
 }
 
 // The block sorts' dynamic shared memory (rows of a tile), above the default limit.
@@ -137,6 +154,42 @@ u64 wide_sort_unique(ra_program* p, const u64* src, int W, u64 n, u64** dst, u64
     return m;
 }
 
+void wide_add_merge(std::vector<WideMergeBatch>& batches, const u64* full, u64 nf, const u64* delta, u64 nd, u64* out,
+                    int W)
+{
+    if (batches.empty() || batches.back().n == kWideJobs) batches.push_back(WideMergeBatch{});
+    WideMergeBatch& mb = batches.back();
+    mb.job[mb.n++] = WideMergeJob{full, delta, out, nullptr, nf, nd, mb.total, mb.tiles, W};
+    mb.total += nd;
+    mb.tiles += ((nf + nd) * (u64)W + kWideMergeTile - 1) / kWideMergeTile;
+}
+
+// The places of the delta rows of some batches' merges, then the merged rows.  Only these two
+// calls use the place scratch.
+void wide_merge_rank(ra_program* p, std::vector<WideMergeBatch>& batches)
+{
+    u64 total = 0;
+    for (const WideMergeBatch& mb : batches) total += mb.total;
+    u64* pos = wide_scratch(p, kWsPlace, total);
+    for (WideMergeBatch& mb : batches) {
+        for (int i = 0; i < mb.n; i++) mb.job[i].pos = pos + mb.job[i].first;
+        pos += mb.total;
+        if (mb.total <= kWideWarpSearch)
+            wide_merge_rank_kernel<true><<<wide_grid(32 * mb.total), kThreads, 0, p->stream>>>(mb);
+        else
+            wide_merge_rank_kernel<false><<<wide_grid(mb.total), kThreads, 0, p->stream>>>(mb);
+        LAUNCHED();
+    }
+}
+
+void wide_merge_copy(ra_program* p, const std::vector<WideMergeBatch>& batches)
+{
+    for (const WideMergeBatch& mb : batches) {
+        wide_merge_copy_kernel<<<(int)std::min<u64>(mb.tiles, kMaxGrid), kThreads, 0, p->stream>>>(mb);
+        LAUNCHED();
+    }
+}
+
 // *a = *a + b (both sorted, in trie order); the merged rows go to the spare
 // buffer, which then becomes *a.
 void wide_merge_into(ra_program* p, Relation& r, u64** a, u64* acap, u64* an, const u64* b, u64 bn)
@@ -151,8 +204,10 @@ void wide_merge_into(ra_program* p, Relation& r, u64** a, u64* acap, u64* an, co
     }
     const u64 n = *an + bn;
     wide_reserve(p, &r.wspare, &r.wspare_cap, n, W, 0);
-    wide_merge_rows_kernel<<<wide_grid(n), kThreads, 0, p->stream>>>(*a, *an, b, bn, W, r.wspare);
-    LAUNCHED();
+    std::vector<WideMergeBatch> one;
+    wide_add_merge(one, *a, *an, b, bn, r.wspare, W);
+    wide_merge_rank(p, one);
+    wide_merge_copy(p, one);
     std::swap(*a, r.wspare);
     std::swap(*acap, r.wspare_cap);
     *an = n;
@@ -360,8 +415,20 @@ void wide_iteration(ra_program* p, Scc& s)
             }
         }
     }
+    // local_insert_in_full's full + delta depends on neither the candidates nor the winners: its
+    // two kernels run while the host waits for those (the host waits for an event before
+    // them), into the spare buffers that become full at the end
+    std::vector<WideMergeBatch> merges;
+    for (int ri : s.rels) {
+        Relation& R = p->rels[ri];
+        if (!R.delta_n) continue;
+        const int W = (int)R.arity + 1;
+        wide_reserve(p, &R.wspare, &R.wspare_cap, R.full_n + R.delta_n, W, 0);
+        wide_add_merge(merges, R.wfull, R.full_n, R.wdelta, R.delta_n, R.wspare, W);
+    }
+    if (!p->wide_ev) CK(cudaEventCreateWithFlags(&p->wide_ev, cudaEventDisableTiming));
     // 1. candidate counts (join ranges, filter passes), one round trip for all rules
-    u64* tot = wide_scratch(p, kWsTot, (u64)nr + outs.size() * (kWideMaxSegs + 2));
+    u64* tot = wide_host_words(p, (u64)nr + outs.size() * (kWideMaxSegs + 2));
     u64* lo = join_rows ? wide_scratch(p, kWsLo, join_rows) : nullptr;
     u64* cnt = join_rows ? wide_scratch(p, kWsCnt, join_rows) : nullptr;
     u64* off = join_rows ? wide_scratch(p, kWsOff, join_rows) : nullptr;
@@ -373,9 +440,21 @@ void wide_iteration(ra_program* p, Scc& s)
         WideCountBatch cb{};
         auto flush_counts = [&]() {
             if (!cb.n) return;
-            wide_count_batch_kernel<<<cb.n, kThreads, 0, p->stream>>>(cb);
+            if (cb.total <= kWideWarpSearch)
+                wide_range_batch_kernel<true><<<wide_grid(32 * cb.total), kThreads, 0, p->stream>>>(cb);
+            else
+                wide_range_batch_kernel<false><<<wide_grid(cb.total), kThreads, 0, p->stream>>>(cb);
             LAUNCHED();
+            wide_count_scan_kernel<<<cb.n, kThreads, 0, p->stream>>>(cb);
+            LAUNCHED();
+            for (int i = 0; i < cb.n; i++) {
+                const WideCountJob& j = cb.job[i];
+                if (j.no <= kWideBlockScan) continue;
+                if (j.pred < 0) wide_scan_async<u64>(p, j.cnt, j.no, j.off, j.total);
+                else wide_scan_async<u32>(p, j.keep, j.no, j.off, j.total);
+            }
             cb.n = 0;
+            cb.total = 0;
         };
         for (int q = 0; q < nr; q++) {
             const Rule& ru = s.rules[q];
@@ -385,33 +464,20 @@ void wide_iteration(ra_program* p, Scc& s)
             const bool join = ru.kind == kJoin;
             const int Wo = join ? (r.pj.left ? r.pj.W0 : r.pj.W1) : (int)p->rels[ru.in0].arity + 1;
             const int Wi = join ? (r.pj.left ? r.pj.W1 : r.pj.W0) : 0;
-            if (r.no <= kWideBlockScan) {   // small: one block of the batched launch
-                WideCountJob& j = cb.job[cb.n++];
-                j = WideCountJob{r.outer, r.inner, r.no, r.ni, join ? lo + r.off : nullptr,
-                                 join ? cnt + r.off : nullptr, join ? off + r.off : pos + r.off,
-                                 join ? nullptr : keep + r.off, tot + q, Wo, Wi, join ? r.pj.jcc : 0,
-                                 join ? -1 : ru.pred};
-                if (cb.n == kWideJobs) flush_counts();
-            } else if (join) {
-                wide_join_count_kernel<<<wide_grid(r.no), kThreads, 0, p->stream>>>(r.outer, Wo, r.no, r.inner, Wi,
-                                                                                    r.ni, r.pj.jcc, lo + r.off,
-                                                                                    cnt + r.off);
-                LAUNCHED();
-                wide_scan_async<u64>(p, cnt + r.off, r.no, off + r.off, tot + q);
-            } else {
-                wide_filter_kernel<<<wide_grid(r.no), kThreads, 0, p->stream>>>(r.outer, Wo, r.no, ru.pred,
-                                                                                keep + r.off);
-                LAUNCHED();
-                wide_scan_async<u32>(p, keep + r.off, r.no, pos + r.off, tot + q);
-            }
+            cb.job[cb.n++] = WideCountJob{r.outer, r.inner, r.no, r.ni, cb.total, join ? lo + r.off : nullptr,
+                                          join ? cnt + r.off : nullptr, join ? off + r.off : pos + r.off,
+                                          join ? nullptr : keep + r.off, tot + q, Wo, Wi, join ? r.pj.jcc : 0,
+                                          join ? -1 : ru.pred};
+            cb.total += r.no;
+            if (cb.n == kWideJobs) flush_counts();
         }
         flush_counts();
+        CK(cudaEventRecord(p->wide_ev, p->stream));
+        wide_merge_rank(p, merges);
         if (counted) {
-            std::vector<u64> h(nr);
-            CK(cudaMemcpyAsync(h.data(), tot, nr * 8, cudaMemcpyDeviceToHost, p->stream));
-            CK(cudaStreamSynchronize(p->stream));
+            CK(cudaEventSynchronize(p->wide_ev));
             for (int q = 0; q < nr; q++)
-                if (rr[q].active && (s.rules[q].kind == kJoin || s.rules[q].kind == RA_COPY_FILTER)) rr[q].total = h[q];
+                if (rr[q].active && (s.rules[q].kind == kJoin || s.rules[q].kind == RA_COPY_FILTER)) rr[q].total = tot[q];
         }
     }
     // 2. candidates into each output relation's buffer, rule by rule, one flattened launch
@@ -503,7 +569,10 @@ void wide_iteration(ra_program* p, Scc& s)
         WideMemberBatch mb{};
         auto flush_member = [&]() {
             if (!mb.n) return;
-            wide_member_batch_kernel<<<wide_grid(mb.total), kThreads, 0, p->stream>>>(mb);
+            if (mb.total <= kWideWarpSearch)
+                wide_member_batch_kernel<true><<<wide_grid(32 * mb.total), kThreads, 0, p->stream>>>(mb);
+            else
+                wide_member_batch_kernel<false><<<wide_grid(mb.total), kThreads, 0, p->stream>>>(mb);
             LAUNCHED();
             mb.n = 0;
             mb.total = 0;
@@ -550,17 +619,15 @@ void wide_iteration(ra_program* p, Scc& s)
             LAUNCHED();
         }
         flush_scan();
-        std::vector<u64> h(outs.size() * (kWideMaxSegs + 2));
-        if (any) {
-            CK(cudaMemcpyAsync(h.data(), picks, h.size() * 8, cudaMemcpyDeviceToHost, p->stream));
-            CK(cudaStreamSynchronize(p->stream));
-        }
+        CK(cudaEventRecord(p->wide_ev, p->stream));
+        wide_merge_copy(p, merges);
+        if (any) CK(cudaEventSynchronize(p->wide_ev));
         for (size_t k = 0; k < outs.size(); k++) {
             WideOut& wo = outs[k];
             Relation& R = p->rels[wo.rel];
             wo.seg_wins.assign(wo.rules.size() + 1, 0);
             if (wo.n) {
-                const u64* my = h.data() + k * (kWideMaxSegs + 2);
+                const u64* my = picks + k * (kWideMaxSegs + 2);
                 for (size_t j = 0; j <= wo.rules.size(); j++) wo.seg_wins[j] = my[j];
                 wo.winners = my[kWideMaxSegs + 1];
             }
@@ -637,37 +704,16 @@ void wide_iteration(ra_program* p, Scc& s)
         }
         flush_newt();
     }
-    // local_insert_in_full: full = full + delta (one flattened launch), delta = newt
+    // local_insert_in_full: full = full + delta (merged above), delta = newt
     {
-        PhaseTimer pt(p, 5);
-        WideMergeBatch mb{};
-        std::vector<int> merged;
-        auto flush_merge = [&]() {
-            if (!mb.n) return;
-            wide_merge_batch_kernel<<<wide_grid(mb.total), kThreads, 0, p->stream>>>(mb);
-            LAUNCHED();
-            for (int ri : merged) {
-                Relation& R = p->rels[ri];
-                std::swap(R.wfull, R.wspare);
-                std::swap(R.wfull_cap, R.wspare_cap);
-                R.full_n += R.delta_n;
-                R.delta_n = 0;
-            }
-            merged.clear();
-            mb.n = 0;
-            mb.total = 0;
-        };
         for (int ri : s.rels) {
             Relation& R = p->rels[ri];
             if (!R.delta_n) continue;
-            const int W = (int)R.arity + 1;
-            wide_reserve(p, &R.wspare, &R.wspare_cap, R.full_n + R.delta_n, W, 0);
-            mb.job[mb.n++] = WideMergeJob{R.wfull, R.wdelta, R.wspare, R.full_n, R.delta_n, mb.total, W};
-            mb.total += R.full_n + R.delta_n;
-            merged.push_back(ri);
-            if (mb.n == kWideJobs) flush_merge();
+            std::swap(R.wfull, R.wspare);
+            std::swap(R.wfull_cap, R.wspare_cap);
+            R.full_n += R.delta_n;
+            R.delta_n = 0;
         }
-        flush_merge();
         for (int ri : s.rels) {
             Relation& R = p->rels[ri];
             std::swap(R.wdelta, R.wnewt);
