@@ -749,6 +749,10 @@ __global__ void __launch_bounds__(kThreads) join_bitmap_kernel(IterCtl* __restri
     __shared__ u64 sm[kWarps + 1];
     if (ctl->flags || ctl->done) return;
     const u64 n = rows_n(ctl, outer_ref);
+    const u64 step = (u64)gridDim.x * kThreads * kBitRows;
+    // blocks past the rows take no part (a thousand arrivals at one counter cost 2 us)
+    const u32 parting = (u32)max((u64)1, min((u64)gridDim.x, (n + kThreads * kBitRows - 1) / (kThreads * kBitRows)));
+    if (blockIdx.x >= parting) return;
     const u64* outer = rows_ptr(ctl, outer_ref);
     const bool filter = ctl->bit_filter != 0;
     const u64 mask = (1ull << bits) - 1;
@@ -757,7 +761,6 @@ __global__ void __launch_bounds__(kThreads) join_bitmap_kernel(IterCtl* __restri
     const int sh1 = ((in1 ? pj.inner_arity : pj.outer_arity) - 1 - pj.col[1]) * bits;
     const int lane = threadIdx.x & 31;
     u64 total = 0;
-    const u64 step = (u64)gridDim.x * kThreads * kBitRows;
     for (u64 base = (u64)blockIdx.x * kThreads * kBitRows; base < n; base += step) {   // block-uniform
         u64 key[kBitRows], s[kBitRows];
         u32 c[kBitRows];
@@ -819,7 +822,7 @@ __global__ void __launch_bounds__(kThreads) join_bitmap_kernel(IterCtl* __restri
     if (threadIdx.x == 0) {
         if (total) atomicAdd((unsigned long long*)&ctl->bit_cand[rule], (unsigned long long)total);
         __threadfence();
-        if (atomicAdd(&ctl->bit_exit[rule], 1u) == gridDim.x - 1) {   // the launch's last block
+        if (atomicAdd(&ctl->bit_exit[rule], 1u) == parting - 1) {   // the launch's last block
             __threadfence();
             ctl->cand_n[rule] = __ldcg((unsigned long long*)&ctl->bit_cand[rule]);
             ctl->bit_cand[rule] = 0;
@@ -979,6 +982,48 @@ __device__ void end_of_iteration(IterCtl* __restrict__ ctl, const SccPlan& plan,
         ctl->heavy_ctr = 0;
     }
     if (use_cond) cudaGraphSetConditional(cond, cont ? 1u : 0u);
+}
+
+// The iteration end by one block, on a copy of the control block in shared memory (`buf`,
+// kEndWords u64): some fifty dependent reads and writes of one thread cost as many L2 round
+// trips in place, 5 to 8 us; here two, to fetch the block and to put it back.  Called by
+// every thread of the launch's last block, when no other block touches the control block
+// any more; tail, when given, decides on the result whether the loop stops for the tail
+// kernel.
+constexpr int kEndWords = (int)(offsetof(IterCtl, bar_count) / 8);
+template <typename Tail>
+__device__ __forceinline__ void end_of_iteration_block(IterCtl* __restrict__ ctl, u64* buf, const SccPlan& plan,
+                                                       const SccRelMap& rm, u64* __restrict__ history,
+                                                       cudaGraphConditionalHandle cond, int use_cond, Tail tail)
+{
+    u64* g = (u64*)ctl;
+    for (int i = threadIdx.x; i < kEndWords; i += kThreads) buf[i] = __ldcg(&g[i]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        IterCtl* L = (IterCtl*)buf;
+        L->exit_ctr = 0;   // the launch is over
+        end_of_iteration(L, plan, rm, history, cond, use_cond);
+        if (use_cond && tail(L)) cudaGraphSetConditional(cond, 0u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kEndWords; i += kThreads) __stcg(&g[i], buf[i]);
+}
+
+// The last of `parting` blocks to get here (after its writes); uniform over the block.
+__device__ __forceinline__ bool last_block(IterCtl* __restrict__ ctl, u32 parting)
+{
+    __shared__ u32 s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&ctl->exit_ctr, 1u) == parting - 1;
+        if (s_last) {
+            __threadfence();
+            atomicExch(&ctl->exit_ctr, 0u);
+        }
+    }
+    __syncthreads();
+    return s_last != 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1202,19 +1247,10 @@ __global__ void __launch_bounds__(kThreads, RA_SELECT_MIN_BLOCKS) select_kernel(
     // blocks past the last tile never write, so only min(grid, tiles) blocks take part
     const u32 parting = (u32)min((u64)gridDim.x, (active && c > 0) ? ntiles : (u64)1);
     if (blockIdx.x >= parting) return;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const u32 done = atomicAdd(&ctl->exit_ctr, 1u);
-        if (done == parting - 1) {
-            __threadfence();
-            ctl->exit_ctr = 0;
-            if (a.last) {
-                end_of_iteration(ctl, plan, rm, history, cond, use_cond);
-                if (a.tail_on && use_cond && tail_next(ctl, a)) cudaGraphSetConditional(cond, 0u);
-            }
-        }
-    }
+    static_assert(kEndWords <= kSelTile, "s_win holds the control block");
+    if (last_block(ctl, parting) && a.last)
+        end_of_iteration_block(ctl, s_win, plan, rm, history, cond, use_cond,
+                               [&](const IterCtl* c) { return a.tail_on && tail_next(c, a); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1251,8 +1287,10 @@ struct BitSelectArgs {
     u64 inst_iter_cap;
 };
 
-__global__ void __launch_bounds__(kThreads) bitmap_select_kernel(IterCtl* __restrict__ ctl, SccPlan plan, SccRelMap rm,
-                                                                 BitSelectArgs a, u64* __restrict__ status,
+__global__ void __launch_bounds__(kThreads) bitmap_select_kernel(IterCtl* __restrict__ ctl,
+                                                                 const __grid_constant__ SccPlan plan,
+                                                                 const __grid_constant__ SccRelMap rm,
+                                                                 const __grid_constant__ BitSelectArgs a, u64* __restrict__ status,
                                                                  u64 status_cap, int tile_slot, u64* __restrict__ history,
                                                                  cudaGraphConditionalHandle cond, int use_cond)
 {
@@ -1262,6 +1300,7 @@ __global__ void __launch_bounds__(kThreads) bitmap_select_kernel(IterCtl* __rest
     __shared__ u64 s_prefix;
     __shared__ u32 s_rows[kWarps][kBitSelRows];     // new tuples of a warp's rows
     __shared__ u64 s_groups[kWarps][kBitSelRows];   // and their groups
+    __shared__ u64 s_end[kEndWords];
     const int out = a.rel, tslot = plan.rule_tag[a.first_rule];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const u64 rows = a.bs.n;
@@ -1390,16 +1429,8 @@ __global__ void __launch_bounds__(kThreads) bitmap_select_kernel(IterCtl* __rest
     }
     const u32 parting = (u32)min((u64)gridDim.x, active ? ntiles : (u64)1);
     if (blockIdx.x >= parting) return;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const u32 done = atomicAdd(&ctl->exit_ctr, 1u);
-        if (done == parting - 1) {
-            __threadfence();
-            ctl->exit_ctr = 0;
-            if (a.last) end_of_iteration(ctl, plan, rm, history, cond, use_cond);
-        }
-    }
+    if (last_block(ctl, parting) && a.last)
+        end_of_iteration_block(ctl, s_end, plan, rm, history, cond, use_cond, [](const IterCtl*) { return false; });
 }
 
 struct SortPassArgs {
@@ -1458,13 +1489,18 @@ __global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict
         const u64 t0 = tile * kSortTile;
         const u32 tn = (u32)min((u64)kSortTile, n - t0);
         // warp w owns items [w*32*IPT, (w+1)*32*IPT) of the tile, round-major = index order
-        u64 kk[kSortIpt];
+        u64 kk[kSortIpt], vv[kSortIpt];
         u32 rk[kSortIpt];
+#pragma unroll
+        for (int r = 0; r < kSortIpt; r++) {   // every load of the tile in flight before the ranking rounds
+            const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
+            kk[r] = li < tn ? a.src_k[t0 + li] : 0;
+            vv[r] = li < tn ? a.src_v[t0 + li] : 0;
+        }
 #pragma unroll
         for (int r = 0; r < kSortIpt; r++) {
             const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
             const bool valid = li < tn;
-            kk[r] = valid ? a.src_k[t0 + li] : 0;
             const int d = valid ? (int)((kk[r] >> a.shift) & (kRadix - 1)) : (kRadix + lane);
             const u32 peers = __match_any_sync(0xffffffffu, d);
             const u32 before = __popc(peers & lanemask_lt());
@@ -1522,7 +1558,7 @@ __global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict
             const int dd = (int)((kk[r] >> a.shift) & (kRadix - 1));
             const u32 pos = s_loc[dd] + s_wcnt[warp][dd] + rk[r];
             s_k[pos] = kk[r];
-            s_v[pos] = a.src_v[t0 + li];
+            s_v[pos] = vv[r];
         }
         __syncthreads();
         // each digit's run is contiguous in the output: coalesced writes
@@ -1659,13 +1695,18 @@ __global__ void __launch_bounds__(kThreads) instance_summary_kernel(
 // ---------------------------------------------------------------------------
 // iteration end as its own launch (reference id order: after the sort passes)
 // ---------------------------------------------------------------------------
-__global__ void iter_end_kernel(IterCtl* __restrict__ ctl, SccPlan plan, SccRelMap rm, u64* __restrict__ history,
-                                cudaGraphConditionalHandle cond, int use_cond)
+__global__ void __launch_bounds__(kThreads) iter_end_kernel(IterCtl* __restrict__ ctl,
+                                                            const __grid_constant__ SccPlan plan,
+                                                            const __grid_constant__ SccRelMap rm,
+                                                            u64* __restrict__ history, cudaGraphConditionalHandle cond,
+                                                            int use_cond)
 {
+    __shared__ u64 s_end[kEndWords];
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < (u64)kMaxSccRels * kMaxPasses * kRadix;
          i += (u64)gridDim.x * blockDim.x)
         (&ctl->sort_hist[0][0][0])[i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) end_of_iteration(ctl, plan, rm, history, cond, use_cond);
+    if (blockIdx.x == 0)
+        end_of_iteration_block(ctl, s_end, plan, rm, history, cond, use_cond, [](const IterCtl*) { return false; });
 }
 
 }  // namespace ra
