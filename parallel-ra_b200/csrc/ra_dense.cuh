@@ -48,6 +48,7 @@ struct DenseArgs {
     int bits;                    // packed column width
     const u64* s_keys;           // S full rows, sorted
     const u64* s_csr;            // S rows with column 0 == v: [s_csr[v], s_csr[v + 1])
+    uint4* s_rec;                // per value: its first seven edges' targets (DenseRec)
     u32* s_edge;                 // per S row: its columns minus its instance's base, column 0 in the upper half
     u64* row_new;                // per row: new tuples
     u64* level_total;            // per iteration: new tuples
@@ -114,6 +115,26 @@ __global__ void __launch_bounds__(kThreads) dense_local_kernel(DenseArgs a, u64 
         } else {
             a.s_edge[j] = (u32)((y - d.base) << 16 | zl);
         }
+    }
+}
+
+// A value's edges in one 16-byte word: u16 number of edges, then the local targets of up to
+// seven (more edges: kRecMany, and the search reads the edge list).  A search step then makes
+// one L2 round trip for a value, where edge range and edges make two.
+constexpr u32 kRecEdges = 7, kRecMany = 0xffffu;
+
+__global__ void __launch_bounds__(kThreads) dense_rec_kernel(DenseArgs a)
+{
+    for (u64 v = (u64)blockIdx.x * kThreads + threadIdx.x; v < a.rows; v += (u64)gridDim.x * kThreads) {
+        const u64 s = a.s_csr[v], c = a.s_csr[v + 1] - s;
+        u32 w[4] = {0, 0, 0, 0};
+        if (c > kRecEdges) {
+            w[0] = kRecMany;
+        } else {
+            w[0] = (u32)c;
+            for (u32 k = 0; k < (u32)c; k++) w[(k + 1) >> 1] |= (a.s_edge[s + k] & 0xffffu) << (((k + 1) & 1) * 16);
+        }
+        a.s_rec[v] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -251,20 +272,34 @@ __device__ __forceinline__ u32 warp_transpose32(u32 x)
     return x;
 }
 
-// z to the end of a block's queue; called by the lanes that have one (any subset of a warp).
-__device__ __forceinline__ void queue_push(u16* q, u32* qn, u32 z)
+// The two queues of a block: entries in shared memory (`near` of each), the rest of a long
+// queue in global memory.
+struct MsQueue {
+    u16* near;
+    u16* far;
+    u32 nnear, nmax;
+    __device__ __forceinline__ u16& at(u32 side, u32 i) const
+    {
+        return i < nnear ? near[side * nnear + i] : far[(u64)side * nmax + i];
+    }
+};
+
+// z to the end of queue `side`; called by the lanes that have one (any subset of a warp).
+__device__ __forceinline__ void queue_push(const MsQueue& q, u32 side, u32* qn, u32 z)
 {
     const u32 m = __activemask();
     const u32 before = __popc(m & lanemask_lt());
     u32 at = 0;
     if (before == 0) at = atomicAdd(qn, (u32)__popc(m));
     at = __shfl_sync(m, at, __ffs(m) - 1);
-    q[at + before] = (u16)z;
+    q.at(side, at + before) = (u16)z;
 }
 
 constexpr int kMsRows = 32;           // rows searched together: one bit each of a value's words
-constexpr u64 kMsMaxN = 19200;        // values per instance: three words of each fit an SM's shared memory
-constexpr u32 kMsSmemQueueN = 13824;  // ... with both queues beside them; above, the queues are in global memory
+constexpr u64 kMsMaxN = 18944;        // values per instance: three words of each fit an SM's shared memory
+constexpr u32 kMsSmemQueueN = 13824;  // ... with both queues beside them; above, kMsNear entries of each are
+constexpr u32 kMsNear = 1024;
+constexpr int kMsWords = 4;           // words of a row a lane loads at a time
 
 // Rows of instances of at most kMsMaxN values: 32 rows of one instance at a time by one
 // CTA, their breadth-first searches run together.  Value z has one word each of known,
@@ -280,7 +315,11 @@ constexpr u32 kMsSmemQueueN = 13824;  // ... with both queues beside them; above
 // 11.5).  Bound by instruction issue and shared-memory conflicts of the random known / next
 // words.  Measured against one warp or CTA per row: n = 16,384, out-degree 2, 3.52 -> 0.97 ms;
 // n = 2,000, 0.24 -> 0.09 ms; the wave's searches 10.0 -> 4.9 ms.
-// Dynamic shared memory: 3 * nmax u32, then (gqueue null) 2 * nmax u16.
+// A narrow level costs one L2 round trip (DenseRec) and two barriers: with edge range, edges and
+// queue each read from L2, and a place in the queue taken for each edge, it took 2.9 us, 2.0 now (n =
+// 16,384, out-degree 1.1, 152 levels:
+// 1.74 -> 1.21 ms).
+// Dynamic shared memory: 3 * nmax u32, then the queues: 2 * (gqueue ? kMsNear : nmax) u16.
 constexpr u32 kMsSweep = 64;
 template <int T>
 __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16* __restrict__ gqueue,
@@ -291,7 +330,8 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
     u32* known = dsm;
     u32* front = dsm + nmax;
     u32* next = dsm + 2 * (u64)nmax;
-    u16* queue = gqueue ? gqueue + (u64)blockIdx.x * 2 * nmax : (u16*)(dsm + 3 * (u64)nmax);
+    const MsQueue queue{(u16*)(dsm + 3 * (u64)nmax), gqueue + (gqueue ? (u64)blockIdx.x * 2 * nmax : 0),
+                        gqueue ? kMsNear : nmax, nmax};
     __shared__ u64 s_chunk;
     __shared__ u32 s_qn[2];
     __shared__ u32 s_lvl[kDenseLevels];   // a chunk's counts stay below 32 * kMsMaxN
@@ -317,22 +357,31 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
         const bool own = lane < (int)ch.count;
         const u32 n = (u32)d.n;
         const u64 e0 = a.s_csr[d.base], e1 = a.s_csr[min(d.base + d.n, a.rows)];   // the instance's edges
-        for (u32 w = warp; w < W; w += T / 32) {
-            const u32 kw = warp_transpose32(own ? krow[w] : 0u);
-            const u32 fw = drow == krow ? kw : warp_transpose32(own ? drow[w] : 0u);
-            const u32 z = w * 32 + lane;
-            known[z] = kw;
-            front[z] = fw;
-            next[z] = 0;
-            if (fw) queue_push(queue, &s_qn[0], z);
-            if (z < n) relax += row_edges(a, d.base + z) * (u64)(long long)(__popc(fw) - __popc(kw));
+        for (u32 w0 = warp; w0 < W; w0 += kMsWords * T / 32) {
+            u32 kw[kMsWords], fw[kMsWords];   // the rows' words, in flight together
+#pragma unroll
+            for (int u = 0; u < kMsWords; u++) {
+                const u32 w = w0 + u * (T / 32);
+                kw[u] = own && w < W ? krow[w] : 0u;
+                fw[u] = drow != krow && own && w < W ? drow[w] : kw[u];
+            }
+#pragma unroll
+            for (int u = 0; u < kMsWords; u++) {
+                const u32 w = w0 + u * (T / 32);
+                if (w >= W) break;   // uniform
+                const u32 k = warp_transpose32(kw[u]), f = drow == krow ? k : warp_transpose32(fw[u]);
+                const u32 z = w * 32 + lane;
+                known[z] = k;
+                front[z] = f;
+                next[z] = 0;
+                if (f) queue_push(queue, 0, &s_qn[0], z);
+                if (z < n) relax += row_edges(a, d.base + z) * (u64)(long long)(__popc(f) - __popc(k));
+            }
         }
         __syncthreads();
         u32 cur = 0, qn = s_qn[0];
         bool queued = true;   // queue `cur` lists the frontier's values
         for (u64 level = 0; qn; level++) {
-            const u16* q = queue + (cur ? nmax : 0);
-            u16* qnext = queue + (cur ? 0 : nmax);
             u32 cnt = 0;
             if (qn >= n / kMsSweep) {
                 queued = false;
@@ -379,25 +428,47 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
                     if (threadIdx.x == 0) s_qn[cur] = 0;
                     __syncthreads();
                     for (u32 z = threadIdx.x; z < W * 32; z += T)
-                        if (front[z]) queue_push(queue + (cur ? nmax : 0), &s_qn[cur], z);
+                        if (front[z]) queue_push(queue, cur, &s_qn[cur], z);
                     queued = true;
                     __syncthreads();
                 }
                 for (u32 i = threadIdx.x; i < qn; i += T) {
-                    const u32 y = q[i];
+                    const u32 y = queue.at(cur, i);
                     const u32 f = front[y];
                     front[y] = 0;
-                    const u64 s = a.s_csr[d.base + y], e = a.s_csr[d.base + y + 1];
-                    for (u64 j = s; j < e; j++) {
-                        const u32 z = a.s_edge[j] & 0xffffu;
-                        const u32 nb = f & ~known[z];
-                        if (nb && atomicOr(&next[z], nb) == 0) queue_push(qnext, &s_qn[cur ^ 1], z);
+                    const uint4 r = d.base + y < a.rows ? a.s_rec[d.base + y] : make_uint4(0, 0, 0, 0);
+                    const u32 c = r.x & 0xffffu;
+                    if (c != kRecMany) {
+                        // all edges' words, then their ORs, then one place in the queue for the values first reached
+                        const u32 w[4] = {r.x, r.y, r.z, r.w};
+                        u32 nb[kRecEdges], first = 0;
+#pragma unroll
+                        for (u32 k = 0; k < kRecEdges; k++)
+                            nb[k] = k < c ? f & ~known[(w[(k + 1) >> 1] >> (((k + 1) & 1) * 16)) & 0xffffu] : 0u;
+#pragma unroll
+                        for (u32 k = 0; k < kRecEdges; k++)
+                            if (nb[k] && atomicOr(&next[(w[(k + 1) >> 1] >> (((k + 1) & 1) * 16)) & 0xffffu], nb[k]) == 0)
+                                first |= 1u << k;
+                        if (first) {
+                            u32 at = atomicAdd(&s_qn[cur ^ 1], (u32)__popc(first));
+#pragma unroll
+                            for (u32 k = 0; k < kRecEdges; k++)
+                                if (first >> k & 1)
+                                    queue.at(cur ^ 1, at++) = (u16)(w[(k + 1) >> 1] >> (((k + 1) & 1) * 16));
+                        }
+                    } else {
+                        const u64 s = a.s_csr[d.base + y], e = a.s_csr[d.base + y + 1];
+                        for (u64 j = s; j < e; j++) {
+                            const u32 z = a.s_edge[j] & 0xffffu;
+                            const u32 nb = f & ~known[z];
+                            if (nb && atomicOr(&next[z], nb) == 0) queue_push(queue, cur ^ 1, &s_qn[cur ^ 1], z);
+                        }
                     }
                 }
                 __syncthreads();
                 const u32 qnew = s_qn[cur ^ 1];
                 for (u32 i = threadIdx.x; i < qnew; i += T) {
-                    const u32 z = qnext[i];
+                    const u32 z = queue.at(cur ^ 1, i);
                     const u32 f = next[z];
                     next[z] = 0;
                     known[z] |= f;
@@ -425,15 +496,25 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
         }
         // the rows' new tuples replace their known bits in global memory
         u32 rcnt = 0;
-        for (u32 w = warp; w < W; w += T / 32) {
-            const u32 z = w * 32 + lane;
-            const u32 kz = known[z];
-            const u32 t = warp_transpose32(kz);
-            if (z < n) relax += row_edges(a, d.base + z) * (u64)__popc(kz);
-            if (own) {
-                const u32 nw = t & ~krow[w];
-                krow[w] = nw;
-                rcnt += __popc(nw);
+        for (u32 w0 = warp; w0 < W; w0 += kMsWords * T / 32) {
+            u32 old[kMsWords];
+#pragma unroll
+            for (int u = 0; u < kMsWords; u++) {
+                const u32 w = w0 + u * (T / 32);
+                old[u] = own && w < W ? krow[w] : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < kMsWords; u++) {
+                const u32 w = w0 + u * (T / 32);
+                if (w >= W) break;
+                const u32 z = w * 32 + lane;
+                const u32 kz = known[z];
+                const u32 nw = warp_transpose32(kz) & ~old[u];
+                if (z < n) relax += row_edges(a, d.base + z) * (u64)__popc(kz);
+                if (own) {
+                    krow[w] = nw;
+                    rcnt += __popc(nw);
+                }
             }
         }
         if (rcnt) atomicAdd(&s_row[lane], rcnt);

@@ -2329,6 +2329,7 @@ struct DenseBufs {
     u64* counters = nullptr;
     u32* flags = nullptr;
     u32* s_edge = nullptr;
+    uint4* s_rec = nullptr;
     DenseInst* inst = nullptr;
     DenseChunk* chunks = nullptr;
     u16* queue = nullptr;
@@ -2343,6 +2344,7 @@ struct DenseBufs {
         dev_free(p, &counters);
         dev_free(p, &flags);
         dev_free(p, &s_edge);
+        dev_free(p, &s_rec);
         dev_free(p, &inst);
         dev_free(p, &chunks);
         dev_free(p, &queue);
@@ -2448,14 +2450,15 @@ bool run_scc_dense(ra_program* p, Scc& s)
     const u64 ms_n[4] = {1024, 4096, kMsSmemQueueN, kMsMaxN};
     typedef void (*DenseMs)(DenseArgs, u32, u16*, const DenseChunk*, u64, u64*);
     const DenseMs ms_all[4] = {dense_ms_kernel<128>, dense_ms_kernel<256>, dense_ms_kernel<512>, dense_ms_kernel<1024>};
-    constexpr u64 kDenseSmemMax = 12 * kMsMaxN;   // 16 * kMsSmemQueueN is less
-    static_assert(16 * kMsSmemQueueN <= kDenseSmemMax && kDenseSmemMax <= 225u << 10, "dynamic shared memory of an SM");
+    constexpr u64 kDenseSmemMax = 12 * kMsMaxN + 4 * kMsNear;   // 16 * kMsSmemQueueN is less
+    static_assert(16 * kMsSmemQueueN <= kDenseSmemMax && kDenseSmemMax + 1024 <= 227u << 10, "dynamic shared memory of an SM");
     CK(cudaMemcpyAsync(B.inst, hi.data(), ninst * sizeof(DenseInst), cudaMemcpyHostToDevice, p->stream));
     const u64 *sk, *sv;
     u64 sn;
     version_rows(p, S, RA_FULL, &sk, &sv, &sn);
     const u64* scsr = version_csr(p, S, RA_FULL);
     dev_alloc(p, &B.s_edge, (sn + 3) & ~3ull);   // read four at a time
+    dev_alloc(p, &B.s_rec, rows);
     const u64 n_stored = R.full_n + R.delta_n;
     u64 level_cap = 256;
     std::vector<u64> hflags(2);
@@ -2483,6 +2486,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
         a.s_keys = sk;
         a.s_csr = scsr;
         a.s_edge = B.s_edge;
+        a.s_rec = B.s_rec;
         a.row_new = B.row_new;
         a.level_total = B.level_total;
         a.inst_level = p->n_inst ? p->dinst_new : nullptr;
@@ -2493,6 +2497,8 @@ bool run_scc_dense(ra_program* p, Scc& s)
             dense_local_kernel<<<grid_for(sn), kThreads, 0, p->stream>>>(a, sn);
             LAUNCHED();
         }
+        dense_rec_kernel<<<grid_for(rows), kThreads, 0, p->stream>>>(a);
+        LAUNCHED();
         if (n_stored) {
             dense_load_kernel<<<grid_for(n_stored), kThreads, 0, p->stream>>>(a, R.keys, R.full_n, n_stored);
             LAUNCHED();
@@ -2542,7 +2548,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
             const void* k = (const void*)dense_closure_kernel;
             if (sh < 4) k = (const void*)(fn[sh] = ms_all[t]);
             smem[sh] = sh == 4 ? 3 * (nmax[sh] / 32) * sizeof(u32)
-                               : (3 * sizeof(u32) + (sh == 3 ? 0 : 2 * sizeof(u16))) * nmax[sh];
+                               : 3 * sizeof(u32) * nmax[sh] + 2 * sizeof(u16) * (sh == 3 ? kMsNear : nmax[sh]);
             if (smem[sh] > 40u << 10)   // the most any launch of this kernel asks for (shapes share kernels)
                 CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmemMax));
             int per_sm = 0;
@@ -2616,7 +2622,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
         }
         dense_emit_kernel<<<std::min<u64>((rows + kWarps - 1) / kWarps, (u64)kSms * 16), kThreads, 0, p->stream>>>(
             DenseArgs{B.inst, p->n_inst ? p->dinst_base : nullptr, ninst, rows, B.known, B.known, p->bits, sk, scsr,
-                      B.s_edge, B.row_new, B.level_total, nullptr, level_cap, B.counters, B.flags},
+                      B.s_rec, B.s_edge, B.row_new, B.level_total, nullptr, level_cap, B.counters, B.flags},
             B.row_off, R.keys + n_stored, R.ids + n_stored, (u64)R.tag << 46, ctr);
         LAUNCHED();
         if (p->kernel_events) {

@@ -121,13 +121,16 @@ def test_bitmap_join_with_deltas_beyond_the_candidate_buffer():
 
 
 # sizes at the edges of the 32-row groups, of the kernel shapes (1,024 / 4,096 / 13,824 values,
-# 19,200 values: above, a row per CTA) and of the wide- and narrow-frontier levels
+# 18,944 values: above, a row per CTA) and of the wide- and narrow-frontier levels
 @pytest.mark.parametrize("n,deg", [(31, 2.0), (32, 1.5), (33, 1.0), (1024, 1.8), (1025, 0.9), (4096, 1.2), (4097, 2.0),
-                                   (13824, 0.9), (13825, 1.15), (19200, 0.95), (19201, 0.9)])
+                                   (13824, 0.9), (13825, 1.15), (18944, 0.95), (18945, 0.9), (16000, 1.6)])
 def test_row_groups_at_shape_edges(n, deg):
     m = round(deg * n)
     rows = er(n, m, n)
     rows[-1, :2] = (n - 1, n // 2)   # the last value is present
+    many = min(12, m // 4)           # one value with more than seven edges
+    rows[:many, 0] = n // 3
+    rows[:many, 1] = np.arange(many)
     pd, rd = run(rows, True)
     assert pd.stats().dense_sccs == 1
     ph, rh = run(rows, False)
