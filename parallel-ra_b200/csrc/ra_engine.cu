@@ -165,8 +165,8 @@ struct ra_program {
     bool packed = false;          // loaded relations packed with `bits` (cleared by a new load)
     bool wide = false;            // this run keeps tuples as rows of u64 columns (ra_wide.cu)
     cudaEvent_t wide_ev = nullptr;   // what the host waits for in a wide iteration
-    u64* hwide = nullptr;         // page-locked counts of a wide iteration (wide_host_words)
-    u64 hwide_cap = 0;
+    u64* hwords = nullptr;        // page-locked words that kernels write counts to (host_words)
+    u64 hwords_cap = 0;
     u64* wbuf[12] = {};           // scratch of the wide path
     u64 wbuf_cap[12] = {};
     bool executed = false;
@@ -571,6 +571,23 @@ void ensure_log(ra_program* p, Relation& r, u64 n)
     grow2(p, &r.keys, &r.ids, &r.cap, n, true, r.full_n + r.delta_n + r.newt_n, p->tune.log_growth);
 }
 
+// Page-locked words that kernels write counts to, for the host to read after its next
+// synchronisation (a copy back costs two extra operations per round trip).
+u64* host_words(ra_program* p, u64 n)
+{
+    if (n > p->hwords_cap) {
+        if (p->hwords) {
+            CK(cudaStreamSynchronize(p->stream));   // nothing still writes the old words
+            cudaFreeHost(p->hwords);
+        }
+        p->hwords = nullptr;
+        p->hwords_cap = 0;
+        CK(cudaMallocHost(&p->hwords, n * 8));
+        p->hwords_cap = n;
+    }
+    return p->hwords;
+}
+
 // ---------------------------------------------------------------------------
 // load: pack raw rows -> sorted, distinct (key, id) rows in the log's full region
 // ---------------------------------------------------------------------------
@@ -583,6 +600,24 @@ void pack_relation(ra_program* p, Relation& r)
     r.delta_version = fresh_stamp();
     if (r.raw_n == 0) return;
     ensure_log(p, r, r.raw_n);
+    if (r.raw_n <= kLoadSmall) {
+        grow2(p, &r.lkeys, &r.lids, &r.l_cap, r.raw_n, false, 0);
+        u64* got = host_words(p, 2);
+        u64 P = 32;
+        while (P < r.raw_n) P <<= 1;
+        CK(cudaFuncSetAttribute(load_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(16 * kLoadSmall)));
+        load_small_kernel<<<1, 1024, 16 * P, p->stream>>>(r.raw, (u32)r.raw_n, (int)r.arity, p->bits, r.keys, r.ids,
+                                                         r.lkeys, r.lids, got);
+        LAUNCHED();
+        CK(cudaStreamSynchronize(p->stream));
+        r.keys_unique = got[1] == 0;
+        (r.version == RA_DELTA ? r.delta_n : r.full_n) = got[0];
+        r.l_n = got[0];
+        r.l_keys_unique = r.keys_unique;
+        r.l_full_stamp = r.full_version;
+        r.l_delta_stamp = r.delta_version;
+        return;
+    }
     rows_pack<<<grid_for(r.raw_n), kThreads, 0, p->stream>>>(r.raw, r.raw_n, (int)r.arity, p->bits, r.keys, r.ids);
     LAUNCHED();
     radix_sort(p, r.keys, r.ids, r.raw_n, 0, key_bits(p, r));
@@ -696,6 +731,14 @@ const u64* version_csr(ra_program* p, Relation& r, int ver)
     const u64 *k, *v;
     u64 n;
     version_rows(p, r, ver, &k, &v, &n);
+    u64& longest = ver == RA_DELTA ? r.csr_delta_longest : r.csr_full_longest;
+    if (nk <= kCsrSmall + 1 && n <= kHeavyRow) {   // no row can be skewed
+        csr_search<<<grid_for(nk), kThreads, 0, p->stream>>>(k, n, (int)(r.arity - r.jcc) * p->bits, nk, *slot);
+        LAUNCHED();
+        longest = n;
+        *stamp = want;
+        return *slot;
+    }
     u32* counts;
     dev_alloc(p, &counts, nk);
     CK(cudaMemsetAsync(counts, 0, nk * 4, p->stream));
@@ -707,7 +750,7 @@ const u64* version_csr(ra_program* p, Relation& r, int ver)
     CK(cudaMemsetAsync(*slot + nk, 0, 8, p->stream));
     csr_row_max<<<grid_for(nk), kThreads, 0, p->stream>>>(counts, nk, (unsigned long long*)(*slot + nk));
     LAUNCHED();
-    (ver == RA_DELTA ? r.csr_delta_longest : r.csr_full_longest) = read_scalar(p, *slot + nk);
+    longest = read_scalar(p, *slot + nk);
     dev_free(p, &counts);
     *stamp = want;
     return *slot;
@@ -1045,7 +1088,7 @@ struct DevRule {
     RowsRef in;            // join: outer rows; copy: input rows
     Projection pj;
     const u64* csr = nullptr;
-    u64 longest = 0;                // join: the inner CSR's longest row (heavy-row split above kHeavyRow)
+    u64 longest = 0;                // join: the inner CSR's longest row if above kHeavyRow (heavy-row split), else 0
     const u64* inner = nullptr;
     int outer_shift = 0;
     int pred = 0;
@@ -1145,7 +1188,8 @@ bool build_dev_scc(ra_program* p, Scc& s, DevScc& d)
             version_rows(p, in, jp.inner_ver, &ik, &iv, &inn);
             dr.inner = ik;
             dr.csr = version_csr(p, in, jp.inner_ver);
-            dr.longest = jp.inner_ver == RA_DELTA ? in.csr_delta_longest : in.csr_full_longest;
+            const u64 longest = jp.inner_ver == RA_DELTA ? in.csr_delta_longest : in.csr_full_longest;
+            dr.longest = longest > kHeavyRow ? longest : 0;   // graphs are kept while it does not matter
             dr.pj = jp.pj;
             const Relation& o = p->rels[jp.outer_rel];
             dr.outer_shift = (int)(o.arity - o.jcc) * p->bits;
@@ -3204,14 +3248,27 @@ void run_scc(ra_program* p, Scc& s)
 
 void choose_bits(ra_program* p)
 {
-    CK(cudaMemsetAsync(p->dscalar + 1, 0, 8, p->stream));
-    for (Relation& r : p->rels)
-        if (r.raw_n) {
+    // small relations: one block each, the values read after one synchronisation
+    u64* got = host_words(p, p->rels.size());
+    bool large = false, small = false;
+    for (size_t i = 0; i < p->rels.size(); i++) {
+        Relation& r = p->rels[i];
+        got[i] = 0;
+        if (!r.raw_n) continue;
+        if (r.raw_n > kLoadSmall) {
+            if (!large) CK(cudaMemsetAsync(p->dscalar + 1, 0, 8, p->stream));
+            large = true;
             rows_max_value<<<grid_for(r.raw_n), kThreads, 0, p->stream>>>(r.raw, r.raw_n, (int)r.arity,
                                                                            p->dscalar + 1);
-            LAUNCHED();
+        } else {
+            small = true;
+            rows_max_small_kernel<<<1, 1024, 0, p->stream>>>(r.raw, (u32)r.raw_n, (int)r.arity, &got[i]);
         }
-    u64 mx = read_scalar(p, p->dscalar + 1);
+        LAUNCHED();
+    }
+    u64 mx = large ? read_scalar(p, p->dscalar + 1) : 0;
+    if (small && !large) CK(cudaStreamSynchronize(p->stream));
+    for (size_t i = 0; i < p->rels.size(); i++) mx = std::max(mx, got[i]);
     int bits = 1;
     while (bits < 64 && (mx >> bits)) bits++;
     // tuples that do not pack into one 63-bit key (or joins the CSR index cannot
@@ -3544,7 +3601,7 @@ int ra_program_destroy(ra_program* p)
         cudaEventDestroy(e.second);
     }
     if (p->stream) cudaStreamSynchronize(p->stream);
-    if (p->hwide) cudaFreeHost(p->hwide);
+    if (p->hwords) cudaFreeHost(p->hwords);
     if (p->wide_ev) cudaEventDestroy(p->wide_ev);
     if (p->hscalar) cudaFreeHost(p->hscalar);
     if (p->hctl) cudaFreeHost(p->hctl);

@@ -67,6 +67,101 @@ __global__ void __launch_bounds__(kThreads) rows_pack(const u64* __restrict__ ro
     }
 }
 
+// Largest data value of a small relation, by one block, straight to page-locked host memory.
+__global__ void __launch_bounds__(1024) rows_max_small_kernel(const u64* __restrict__ rows, u32 n, int arity,
+                                                              u64* __restrict__ host_out)
+{
+    __shared__ u64 s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    const u32 w = (u32)arity + 1;
+    u64 m = 0;
+    for (u32 e = threadIdx.x; e < n * w; e += blockDim.x)
+        if (e % w != (u32)arity) m = max(m, rows[e]);
+    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if ((threadIdx.x & 31) == 0) atomicMax((unsigned long long*)&s_max, (unsigned long long)m);
+    __syncthreads();
+    if (threadIdx.x == 0) *host_out = s_max;
+}
+
+// The whole load of a small relation by one block: rows packed, sorted by (key, id) in shared
+// memory (bitonic; 16 bytes per row), exact repetitions dropped, the result written to the log
+// and to the copy that a reset restores; row count and whether two rows share data columns go
+// straight to page-locked host memory.  A radix sort takes five launches per 8 key bits and two
+// round trips here; bound by the network's stages.  Up to kLoadSmall rows: measured LDSM.
+constexpr u32 kLoadSmall = 8192;
+__global__ void __launch_bounds__(1024) load_small_kernel(const u64* __restrict__ rows, u32 n, int arity, int bits,
+                                                          u64* __restrict__ keys, u64* __restrict__ ids,
+                                                          u64* __restrict__ lkeys, u64* __restrict__ lids,
+                                                          u64* __restrict__ host_out)
+{
+    extern __shared__ u64 l_rows[];
+    __shared__ u64 sm[33];
+    __shared__ u32 s_dup;
+    u32 P = 32;
+    while (P < n) P <<= 1;
+    u64* k = l_rows;
+    u64* v = l_rows + P;
+    const u32 T = blockDim.x, t = threadIdx.x, w = (u32)arity + 1;
+    if (t == 0) s_dup = 0;
+    for (u32 i = t; i < P; i += T) {
+        u64 key = ~0ull, id = ~0ull;   // padding: above every packed key
+        if (i < n) {
+            key = 0;
+            for (int c = 0; c < arity; c++) key = (key << bits) | rows[i * w + c];
+            id = rows[i * w + arity];
+        }
+        k[i] = key;
+        v[i] = id;
+    }
+    __syncthreads();
+    for (u32 len = 2; len <= P; len <<= 1) {
+        for (u32 j = len >> 1; j > 0; j >>= 1) {
+            for (u32 p = t; p < P / 2; p += T) {   // a thread per pair
+                const u32 lo = 2 * p - (p & (j - 1)), hi = lo + j;
+                const u64 ka = k[lo], kb = k[hi], va = v[lo], vb = v[hi];
+                const bool after = ka > kb || (ka == kb && va > vb);
+                if (after == ((lo & len) == 0)) {
+                    k[lo] = kb;
+                    k[hi] = ka;
+                    v[lo] = vb;
+                    v[hi] = va;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // distinct rows, consecutive ones per thread
+    const u32 per = (n + T - 1) / T, b = min(n, t * per), e = min(n, b + per);
+    u64 kept = 0;
+    for (u32 i = b; i < e; i++) {
+        const bool same = i && k[i] == k[i - 1];
+        if (same) s_dup = 1;
+        kept += !(same && v[i] == v[i - 1]);
+    }
+    // exclusive scan over the block's 32 warps
+    const u64 inc = warp_inclusive_scan(kept);
+    if ((t & 31) == 31) sm[t >> 5] = inc;
+    __syncthreads();
+    if (t < 32) {
+        const u64 x = t < T / 32 ? sm[t] : 0, xi = warp_inclusive_scan(x);
+        sm[t] = xi - x;
+        if (t == 31) sm[32] = xi;
+    }
+    __syncthreads();
+    u64 at = inc - kept + sm[t >> 5];
+    for (u32 i = b; i < e; i++) {
+        if (i && k[i] == k[i - 1] && v[i] == v[i - 1]) continue;
+        keys[at] = lkeys[at] = k[i];
+        ids[at] = lids[at] = v[i];
+        at++;
+    }
+    if (t == 0) {
+        host_out[0] = sm[32];
+        host_out[1] = s_dup;
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) rows_unpack(const u64* __restrict__ keys, const u64* __restrict__ ids,
                                                         u64 n, int arity, int bits, u64* __restrict__ rows)
 {
@@ -117,6 +212,23 @@ __global__ void __launch_bounds__(kThreads) csr_count(const u64* __restrict__ ke
 {
     for (u64 i = (u64)blockIdx.x * kThreads + threadIdx.x; i < n; i += (u64)gridDim.x * kThreads)
         atomicAdd(&counts[keys[i] >> shift], 1u);
+}
+
+// The offsets themselves for a small key range, a thread per offset: the first of the sorted
+// rows whose join key is not below it (one launch where counting and scanning take five).
+constexpr u64 kCsrSmall = 1ull << 16;
+__global__ void __launch_bounds__(kThreads) csr_search(const u64* __restrict__ keys, u64 n, int shift, u64 nk,
+                                                       u64* __restrict__ offsets)
+{
+    for (u64 j = (u64)blockIdx.x * kThreads + threadIdx.x; j < nk; j += (u64)gridDim.x * kThreads) {
+        u64 lo = 0, hi = n;
+        while (lo < hi) {
+            const u64 m = (lo + hi) >> 1;
+            if ((keys[m] >> shift) < j) lo = m + 1;
+            else hi = m;
+        }
+        offsets[j] = lo;
+    }
 }
 
 // The longest CSR row (most rows sharing one join key), stored after the offsets:

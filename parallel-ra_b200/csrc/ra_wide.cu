@@ -74,23 +74,6 @@ void wide_reserve32(ra_program* p, u32** buf, u64* cap, u64 n)
 
 int wide_grid(u64 n) { return grid_for(std::max<u64>(n, 1)); }
 
-// Page-locked words that kernels write an iteration's counts to, for the host to read after
-// its next synchronisation (a copy back costs two extra operations per round trip).
-u64* wide_host_words(ra_program* p, u64 n)
-{
-    if (n > p->hwide_cap) {
-        if (p->hwide) {
-            CK(cudaStreamSynchronize(p->stream));   // nothing still writes the old words
-            cudaFreeHost(p->hwide);
-        }
-        p->hwide = nullptr;
-        p->hwide_cap = 0;
-        CK(cudaMallocHost(&p->hwide, n * 8));
-        p->hwide_cap = n;
-    }
-    return p->hwide;
-}
-
 // Exclusive scan of n values into out, the total into *total (device or page-locked), with
 // no host round trip (one block for small inputs).
 template <typename T>
@@ -428,7 +411,7 @@ void wide_iteration(ra_program* p, Scc& s)
     }
     if (!p->wide_ev) CK(cudaEventCreateWithFlags(&p->wide_ev, cudaEventDisableTiming));
     // 1. candidate counts (join ranges, filter passes), one round trip for all rules
-    u64* tot = wide_host_words(p, (u64)nr + outs.size() * (kWideMaxSegs + 2));
+    u64* tot = host_words(p, (u64)nr + outs.size() * (kWideMaxSegs + 2));
     u64* lo = join_rows ? wide_scratch(p, kWsLo, join_rows) : nullptr;
     u64* cnt = join_rows ? wide_scratch(p, kWsCnt, join_rows) : nullptr;
     u64* off = join_rows ? wide_scratch(p, kWsOff, join_rows) : nullptr;
