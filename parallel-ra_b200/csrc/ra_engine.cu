@@ -171,7 +171,8 @@ struct ra_program {
     u64 wbuf_cap[12] = {};
     bool executed = false;
     bool running = false;         // between the first and the last SCC of a run
-    double fixpoint_ms_acc = 0;
+    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> scc_ev;   // around each SCC of the run
+    size_t scc_ev_n = 0;
     u64 epoch = 0;
     std::string err;
     ra_stats stats{};
@@ -202,7 +203,6 @@ struct ra_program {
     u64 hist_cap = 0;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> dedup_events;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> phase_events;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // device-driven SCC runs (graph mode)
     IterCtl* ctl = nullptr;
     IterCtl* hctl = nullptr;      // pinned mirror (header part)
@@ -483,7 +483,7 @@ void rows_to_host(ra_program* p, void* dst, const void* src, u64 bytes)
 // exclusive scan of n values into out (u64); returns the total (synchronises)
 // ---------------------------------------------------------------------------
 template <typename T>
-u64 scan_exclusive(ra_program* p, const T* in, u64 n, u64* out, bool want_total = true)
+u64 scan_exclusive(ra_program* p, const T* in, u64 n, u64* out, bool want_total = true, u64* total = nullptr)
 {
     if (n == 0) return 0;
     int g = grid_for(n);
@@ -492,7 +492,7 @@ u64 scan_exclusive(ra_program* p, const T* in, u64 n, u64* out, bool want_total 
     g = (int)((n + chunk - 1) / chunk);
     scan_chunk_sums<T><<<g, kThreads, 0, p->stream>>>(in, n, chunk, p->sums);
     LAUNCHED();
-    scan_sums_single<<<1, kThreads, 0, p->stream>>>(p->sums, g, p->dscalar);
+    scan_sums_single<<<1, kThreads, 0, p->stream>>>(p->sums, g, total ? total : p->dscalar);
     LAUNCHED();
     scan_chunk_apply<T><<<g, kThreads, 0, p->stream>>>(in, n, chunk, p->sums, out);
     LAUNCHED();
@@ -2111,8 +2111,8 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
         ensure_log(p, r, base + std::max<u64>(base, 1u << 20));
     }
     refresh_refs(p, d);
-    CK(cudaMemcpyAsync(p->ctl, p->hctl, ctl_header_bytes(), cudaMemcpyHostToDevice, p->stream));
-    CK(cudaMemsetAsync(&p->ctl->sort_hist[0][0][0], 0, sizeof(p->ctl->sort_hist), p->stream));
+    if (p->id_order == RA_IDS_REFERENCE)
+        CK(cudaMemsetAsync(&p->ctl->sort_hist[0][0][0], 0, sizeof(p->ctl->sort_hist), p->stream));
     u64 outer0 = 0;
     for (const DevRule& r : d.rules) outer0 = std::max(outer0, r.in.slot >= 0 ? p->rels[d.rel_of_slot[r.in.slot]].delta_n : r.in.static_n);
     for (u64 want = std::max<u64>({p->dcand_cap, 1u << 22, 2 * outer0});; want /= 2) {
@@ -2128,7 +2128,7 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
         }
     }
     CK(cudaMemsetAsync(p->status, 0, p->status_cap * 8, p->stream));
-    CK(cudaMemcpyAsync(&p->ctl->time_cap, &p->hctl->time_cap, 8, cudaMemcpyHostToDevice, p->stream));
+    CK(cudaMemcpyAsync(p->ctl, p->hctl, ctl_header_bytes(), cudaMemcpyHostToDevice, p->stream));
     if (p->n_inst) {
         size_instance_rows(p, 256);
         CK(cudaMemsetAsync(p->dinst_new, 0, p->inst_rows_cap * p->n_inst * 8, p->stream));
@@ -2300,15 +2300,22 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
     std::vector<u64> hist(2 * h.hist_n);
     const u64 nt = std::min<u64>(h.iteration, p->dhist_cap);
     std::vector<u64> ends(nt);
-    if (h.hist_n) CK(cudaMemcpyAsync(hist.data(), p->dhist, 2 * h.hist_n * 8, cudaMemcpyDeviceToHost, p->stream));
-    if (nt) CK(cudaMemcpyAsync(ends.data(), p->dhist + 2 * p->dhist_cap, nt * 8, cudaMemcpyDeviceToHost, p->stream));
+    if (h.hist_n == 1 && nt == 1) {   // came with the control block
+        hist[0] = h.last_delta;
+        hist[1] = h.last_full;
+        ends[0] = h.last_time;
+    } else {
+        if (h.hist_n) CK(cudaMemcpyAsync(hist.data(), p->dhist, 2 * h.hist_n * 8, cudaMemcpyDeviceToHost, p->stream));
+        if (nt) CK(cudaMemcpyAsync(ends.data(), p->dhist + 2 * p->dhist_cap, nt * 8, cudaMemcpyDeviceToHost, p->stream));
+        if (h.hist_n || nt) CK(cudaStreamSynchronize(p->stream));
+    }
     if (p->n_inst && h.iteration) {
         const size_t at = p->inst_hist.size();
         p->inst_hist.resize(at + (size_t)h.iteration * p->n_inst);
         CK(cudaMemcpyAsync(p->inst_hist.data() + at, p->dinst_new, (size_t)h.iteration * p->n_inst * 8,
                            cudaMemcpyDeviceToHost, p->stream));
+        CK(cudaStreamSynchronize(p->stream));
     }
-    CK(cudaStreamSynchronize(p->stream));
     {
         u64 prev = h.t_start;
         for (u64 i = 0; i < nt; i++) {
@@ -2365,35 +2372,33 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
 // Device buffers of one dense evaluation, freed on every exit.
 struct DenseBufs {
     ra_program* p;
+    u8* all = nullptr;      // one allocation, cut into the arrays below
+    u64 used = 0;
     u32* known = nullptr;
     u32* delta0 = nullptr;
     u64* row_new = nullptr;
     u64* row_off = nullptr;
-    u64* level_total = nullptr;
-    u64* counters = nullptr;
-    u32* flags = nullptr;
     u32* s_edge = nullptr;
     uint4* s_rec = nullptr;
     DenseInst* inst = nullptr;
     DenseChunk* chunks = nullptr;
     u16* queue = nullptr;
+    u64* meta = nullptr;    // flags, total, counters, level totals: read back together
     explicit DenseBufs(ra_program* pp) : p(pp) {}
     ~DenseBufs()
     {
-        dev_free(p, &known);
-        dev_free(p, &delta0);
-        dev_free(p, &row_new);
-        dev_free(p, &row_off);
-        dev_free(p, &level_total);
-        dev_free(p, &counters);
-        dev_free(p, &flags);
-        dev_free(p, &s_edge);
-        dev_free(p, &s_rec);
-        dev_free(p, &inst);
-        dev_free(p, &chunks);
-        dev_free(p, &queue);
+        dev_free(p, &all);
+        dev_free(p, &meta);
+    }
+    // room for count Ts in the allocation: with `all` set, their address
+    template <typename T>
+    void cut(T** at, u64 count)
+    {
+        if (all) *at = (T*)(all + used);
+        used += (count * sizeof(T) + 255) & ~255ull;
     }
 };
+constexpr u64 kDenseTotal = 1, kDenseCounters = 2, kDenseLevels0 = 10;   // words of DenseBufs::meta; flags in word 0
 
 // The end of a closure-shaped SCC run by an evaluator that is not the iteration
 // loop (dense rows, composed reachable sets): `total` new tuples already written
@@ -2479,15 +2484,6 @@ bool run_scc_dense(ra_program* p, Scc& s)
     }
     if (2.0 * 4.0 * (double)words + 16.0 * (double)rows > p->tune.dense_max_bytes) return false;
 
-    DenseBufs B(p);
-    const bool all_delta = R.full_n == 0;   // every stored tuple is in the initial delta: one matrix holds both
-    dev_alloc(p, &B.known, words);
-    if (!all_delta) dev_alloc(p, &B.delta0, words);
-    dev_alloc(p, &B.row_new, rows);
-    dev_alloc(p, &B.row_off, rows);
-    dev_alloc(p, &B.counters, 8);
-    dev_alloc(p, &B.flags, 1);
-    dev_alloc(p, &B.inst, ninst);
     // the searches: 32 rows of an instance per CTA (dense_ms_kernel) in four shapes by the
     // instance's values, or one row per CTA (dense_closure_kernel) above kMsMaxN values
     constexpr int kShapes = 5;
@@ -2495,30 +2491,97 @@ bool run_scc_dense(ra_program* p, Scc& s)
     typedef void (*DenseMs)(DenseArgs, u32, u16*, const DenseChunk*, u64, u64*);
     const DenseMs ms_all[4] = {dense_ms_kernel<128>, dense_ms_kernel<256>, dense_ms_kernel<512>, dense_ms_kernel<1024>};
     constexpr u64 kDenseSmemMax = 12 * kMsMaxN + 4 * kMsNear;   // 16 * kMsSmemQueueN is less
-    static_assert(16 * kMsSmemQueueN <= kDenseSmemMax && kDenseSmemMax + 1024 <= 227u << 10, "dynamic shared memory of an SM");
-    CK(cudaMemcpyAsync(B.inst, hi.data(), ninst * sizeof(DenseInst), cudaMemcpyHostToDevice, p->stream));
+    static_assert(16 * kMsSmemQueueN <= kDenseSmemMax && kDenseSmemMax + 1024 <= 227u << 10,
+                  "dynamic shared memory of an SM");
+    // work: chunks of rows of one instance, the widest instances first
+    auto shape_of = [&](u32 i) {
+        int sh = 0;
+        while (sh < 4 && hi[i].n > ms_n[sh]) sh++;
+        return sh;
+    };
+    std::vector<u32> order(ninst);
+    for (u32 i = 0; i < ninst; i++) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](u32 x, u32 y) { return hi[x].n > hi[y].n; });
+    std::vector<DenseChunk> chunks;
+    u64 first[kShapes + 1] = {0};
+    u64 nmax[kShapes] = {0};
+    for (int sh = 0; sh < kShapes; sh++) {
+        first[sh] = chunks.size();
+        for (u32 i : order) {
+            const DenseInst& di = hi[i];
+            if (shape_of(i) != sh || di.base >= rows) continue;
+            nmax[sh] = std::max(nmax[sh], (di.n + 31) / 32 * 32);
+            const u64 cnt = std::min(di.n, rows - di.base), per = sh == 4 ? 4 : kMsRows;
+            for (u64 r0 = 0; r0 < cnt; r0 += per)
+                chunks.push_back(DenseChunk{di.base + r0, i, (u32)std::min(per, cnt - r0)});
+        }
+    }
+    first[kShapes] = chunks.size();
+    // grids: resident CTAs of each kernel, at most one per chunk
+    u64 nc[kShapes];
+    DenseMs fn[4] = {nullptr, nullptr, nullptr, nullptr};
+    size_t smem[kShapes];
+    int grids[kShapes], threads[kShapes];
+    for (int sh = 0; sh < kShapes; sh++) {
+        nc[sh] = first[sh + 1] - first[sh];
+        if (!nc[sh]) continue;
+        // threads per CTA: as many as its values when the chunks leave SMs idle, else several CTAs per SM
+        const bool few = nc[sh] <= (u64)kSms;
+        const int t = sh >= 2 ? 3 : sh == 1 ? (few ? 3 : 1) : (few ? (nmax[sh] > 256 ? 2 : 1) : 0);
+        threads[sh] = sh == 4 ? kThreads : 128 << t;
+        const void* k = (const void*)dense_closure_kernel;
+        if (sh < 4) k = (const void*)(fn[sh] = ms_all[t]);
+        smem[sh] = sh == 4 ? 3 * (nmax[sh] / 32) * sizeof(u32)
+                           : 3 * sizeof(u32) * nmax[sh] + 2 * sizeof(u16) * (sh == 3 ? kMsNear : nmax[sh]);
+        if (smem[sh] > 40u << 10)   // the most any launch of this kernel asks for (shapes share kernels)
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmemMax));
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads[sh], smem[sh]));
+        grids[sh] = (int)std::max<u64>(1, std::min((u64)kSms * (u64)std::max(per_sm, 1), nc[sh]));
+    }
+
     const u64 *sk, *sv;
     u64 sn;
     version_rows(p, S, RA_FULL, &sk, &sv, &sn);
     const u64* scsr = version_csr(p, S, RA_FULL);
-    dev_alloc(p, &B.s_edge, (sn + 3) & ~3ull);   // read four at a time
-    dev_alloc(p, &B.s_rec, rows);
+    const bool all_delta = R.full_n == 0;   // every stored tuple is in the initial delta: one matrix holds both
+    DenseBufs B(p);
+    for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
+        if (pass) {
+            dev_alloc(p, &B.all, B.used);
+            B.used = 0;
+        }
+        B.cut(&B.known, words);
+        if (!all_delta) B.cut(&B.delta0, words);
+        B.cut(&B.row_new, rows);
+        B.cut(&B.row_off, rows);
+        B.cut(&B.s_rec, rows);
+        B.cut(&B.s_edge, (sn + 3) & ~3ull);   // read four at a time
+        B.cut(&B.inst, ninst);
+        B.cut(&B.chunks, std::max<size_t>(chunks.size(), 1));
+        if (nc[3]) B.cut(&B.queue, (u64)grids[3] * 2 * nmax[3]);
+    }
+    CK(cudaMemcpyAsync(B.inst, hi.data(), ninst * sizeof(DenseInst), cudaMemcpyHostToDevice, p->stream));
+    if (!chunks.empty())
+        CK(cudaMemcpyAsync(B.chunks, chunks.data(), chunks.size() * sizeof(DenseChunk), cudaMemcpyHostToDevice,
+                           p->stream));
     const u64 n_stored = R.full_n + R.delta_n;
     u64 level_cap = 256;
-    std::vector<u64> hflags(2);
+    u64* got = nullptr;   // meta, read back
     for (;;) {
-        dev_free(p, &B.level_total);
-        dev_alloc(p, &B.level_total, level_cap);
         if (p->n_inst) {
             size_instance_rows(p, level_cap);
+            level_cap = std::min(level_cap, p->inst_rows_cap);
             CK(cudaMemsetAsync(p->dinst_new, 0, p->inst_rows_cap * p->n_inst * 8, p->stream));
         }
+        dev_free(p, &B.meta);
+        dev_alloc(p, &B.meta, kDenseLevels0 + level_cap);
+        u64* counters = B.meta + kDenseCounters;
+        CK(cudaMemsetAsync(B.meta, 0, (kDenseLevels0 + level_cap) * 8, p->stream));
         CK(cudaMemsetAsync(B.known, 0, words * 4, p->stream));
         if (!all_delta) CK(cudaMemsetAsync(B.delta0, 0, words * 4, p->stream));
-        CK(cudaMemsetAsync(B.row_new, 0, rows * 8, p->stream));
-        CK(cudaMemsetAsync(B.level_total, 0, level_cap * 8, p->stream));
-        CK(cudaMemsetAsync(B.counters, 0, 8 * 8, p->stream));
-        CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
+        // the 32-row searches write every row's count; values below the first instance have no search
+        if (nc[4] || hi[0].base) CK(cudaMemsetAsync(B.row_new, 0, rows * 8, p->stream));
         DenseArgs a{};
         a.inst = B.inst;
         a.inst_base = p->n_inst ? p->dinst_base : nullptr;
@@ -2532,11 +2595,11 @@ bool run_scc_dense(ra_program* p, Scc& s)
         a.s_edge = B.s_edge;
         a.s_rec = B.s_rec;
         a.row_new = B.row_new;
-        a.level_total = B.level_total;
+        a.level_total = B.meta + kDenseLevels0;
         a.inst_level = p->n_inst ? p->dinst_new : nullptr;
-        a.level_cap = p->n_inst ? std::min(level_cap, p->inst_rows_cap) : level_cap;
-        a.counters = B.counters;
-        a.flags = B.flags;
+        a.level_cap = level_cap;
+        a.counters = counters;
+        a.flags = (u32*)B.meta;
         if (sn) {
             dense_local_kernel<<<grid_for(sn), kThreads, 0, p->stream>>>(a, sn);
             LAUNCHED();
@@ -2547,62 +2610,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
             dense_load_kernel<<<grid_for(n_stored), kThreads, 0, p->stream>>>(a, R.keys, R.full_n, n_stored);
             LAUNCHED();
         }
-        // work: chunks of rows of one instance, the widest instances first
-        auto shape_of = [&](u32 i) {
-            int sh = 0;
-            while (sh < 4 && hi[i].n > ms_n[sh]) sh++;
-            return sh;
-        };
-        std::vector<u32> order(ninst);
-        for (u32 i = 0; i < ninst; i++) order[i] = i;
-        std::stable_sort(order.begin(), order.end(), [&](u32 x, u32 y) { return hi[x].n > hi[y].n; });
-        std::vector<DenseChunk> chunks;
-        u64 first[kShapes + 1] = {0};
-        u64 nmax[kShapes] = {0};
-        for (int sh = 0; sh < kShapes; sh++) {
-            first[sh] = chunks.size();
-            for (u32 i : order) {
-                const DenseInst& di = hi[i];
-                if (shape_of(i) != sh || di.base >= rows) continue;
-                nmax[sh] = std::max(nmax[sh], (di.n + 31) / 32 * 32);
-                const u64 cnt = std::min(di.n, rows - di.base), per = sh == 4 ? 4 : kMsRows;
-                for (u64 r0 = 0; r0 < cnt; r0 += per)
-                    chunks.push_back(DenseChunk{di.base + r0, i, (u32)std::min(per, cnt - r0)});
-            }
-        }
-        first[kShapes] = chunks.size();
-        dev_free(p, &B.chunks);
-        dev_alloc(p, &B.chunks, std::max<size_t>(chunks.size(), 1));
-        if (!chunks.empty())
-            CK(cudaMemcpyAsync(B.chunks, chunks.data(), chunks.size() * sizeof(DenseChunk), cudaMemcpyHostToDevice,
-                               p->stream));
-        // grids: resident CTAs of each kernel, at most one per chunk
-        u64* ctr[kShapes] = {B.counters + 2, B.counters + 3, B.counters + 4, B.counters + 7, B.counters};
-        u64 nc[kShapes];
-        DenseMs fn[4] = {nullptr, nullptr, nullptr, nullptr};
-        size_t smem[kShapes];
-        int grids[kShapes], threads[kShapes];
-        for (int sh = 0; sh < kShapes; sh++) {
-            nc[sh] = first[sh + 1] - first[sh];
-            if (!nc[sh]) continue;
-            // threads per CTA: as many as its values when the chunks leave SMs idle, else several CTAs per SM
-            const bool few = nc[sh] <= (u64)kSms;
-            const int t = sh >= 2 ? 3 : sh == 1 ? (few ? 3 : 1) : (few ? (nmax[sh] > 256 ? 2 : 1) : 0);
-            threads[sh] = sh == 4 ? kThreads : 128 << t;
-            const void* k = (const void*)dense_closure_kernel;
-            if (sh < 4) k = (const void*)(fn[sh] = ms_all[t]);
-            smem[sh] = sh == 4 ? 3 * (nmax[sh] / 32) * sizeof(u32)
-                               : 3 * sizeof(u32) * nmax[sh] + 2 * sizeof(u16) * (sh == 3 ? kMsNear : nmax[sh]);
-            if (smem[sh] > 40u << 10)   // the most any launch of this kernel asks for (shapes share kernels)
-                CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmemMax));
-            int per_sm = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads[sh], smem[sh]));
-            grids[sh] = (int)std::max<u64>(1, std::min((u64)kSms * (u64)std::max(per_sm, 1), nc[sh]));
-        }
-        if (nc[3]) {
-            dev_free(p, &B.queue);
-            dev_alloc(p, &B.queue, (u64)grids[3] * 2 * nmax[3]);
-        }
+        u64* ctr[kShapes] = {counters + 2, counters + 3, counters + 4, counters + 7, counters};
         cudaEvent_t ev[2] = {nullptr, nullptr};
         if (p->kernel_events) {
             CK(cudaEventCreate(&ev[0]));
@@ -2627,13 +2635,17 @@ bool run_scc_dense(ra_program* p, Scc& s)
             cudaEventDestroy(ev[0]);
             cudaEventDestroy(ev[1]);
         }
-        u32 fl = 0;
-        CK(cudaMemcpyAsync(&fl, B.flags, 4, cudaMemcpyDeviceToHost, p->stream));
+        // every row's first output, the total with the flags, counters and levels: one round trip
+        if (rows <= (u64)kThreads * kWideScanPer)
+            wide_scan_small_kernel<u64><<<1, kThreads, 0, p->stream>>>(B.row_new, rows, B.row_off, B.meta + kDenseTotal);
+        else
+            scan_exclusive<u64>(p, B.row_new, rows, B.row_off, false, B.meta + kDenseTotal);
+        got = host_words(p, kDenseLevels0 + level_cap);
+        CK(cudaMemcpyAsync(got, B.meta, (kDenseLevels0 + level_cap) * 8, cudaMemcpyDeviceToHost, p->stream));
         CK(cudaStreamSynchronize(p->stream));
+        const u32 fl = (u32)got[0];
         if (fl & kDenseFlagRange) {
-            u64 bad[2] = {0, 0};
-            CK(cudaMemcpyAsync(bad, B.counters + 5, 16, cudaMemcpyDeviceToHost, p->stream));
-            CK(cudaStreamSynchronize(p->stream));
+            const u64 bad[2] = {got[kDenseCounters + 5], got[kDenseCounters + 6]};
             const u64 key = bad[0] - 1, mask = (1ull << p->bits) - 1;
             const u64 c0 = (key >> p->bits) & mask, c1 = key & mask;
             // R's rows are keyed by column 1's instance, S's by column 0's
@@ -2645,16 +2657,13 @@ bool run_scc_dense(ra_program* p, Scc& s)
                  s.id, (unsigned long long)c0, (unsigned long long)c1, bad[1] == 1 ? R.name.c_str() : S.name.c_str(),
                  inst, (unsigned long long)hi[inst].base, (unsigned long long)(hi[inst].base + hi[inst].n - 1));
         }
-        if (!(fl & kDenseFlagLevels)) {
-            level_cap = a.level_cap;
-            break;
-        }
+        if (!(fl & kDenseFlagLevels)) break;
         level_cap *= 4;   // a deeper search than the level arrays held: again with room
         p->stats.regrows++;
     }
 
     // new tuples, row by row, after R's stored ones
-    const u64 total = scan_exclusive<u64>(p, B.row_new, rows, B.row_off);
+    const u64 total = got[kDenseTotal];
     u64& ctr = intern_counter(p, R.tag);
     if (total) {
         ensure_log(p, R, n_stored + total);
@@ -2666,7 +2675,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
         }
         dense_emit_kernel<<<std::min<u64>((rows + kWarps - 1) / kWarps, (u64)kSms * 16), kThreads, 0, p->stream>>>(
             DenseArgs{B.inst, p->n_inst ? p->dinst_base : nullptr, ninst, rows, B.known, B.known, p->bits, sk, scsr,
-                      B.s_rec, B.s_edge, B.row_new, B.level_total, nullptr, level_cap, B.counters, B.flags},
+                      B.s_rec, B.s_edge, B.row_new, nullptr, nullptr, level_cap, nullptr, nullptr},
             B.row_off, R.keys + n_stored, R.ids + n_stored, (u64)R.tag << 46, ctr);
         LAUNCHED();
         if (p->kernel_events) {
@@ -2679,10 +2688,8 @@ bool run_scc_dense(ra_program* p, Scc& s)
             cudaEventDestroy(ev[1]);
         }
     }
-    std::vector<u64> lv(level_cap), cnt(4);
-    CK(cudaMemcpyAsync(lv.data(), B.level_total, level_cap * 8, cudaMemcpyDeviceToHost, p->stream));
-    CK(cudaMemcpyAsync(cnt.data(), B.counters, 4 * 8, cudaMemcpyDeviceToHost, p->stream));
-    CK(cudaStreamSynchronize(p->stream));
+    const std::vector<u64> lv(got + kDenseLevels0, got + kDenseLevels0 + level_cap);
+    const u64 visited = got[kDenseCounters + 1];
     u64 L = 0;
     while (L < level_cap && lv[L]) L++;
     const u64 iterations = L + 1;   // the last one finds nothing new
@@ -2695,7 +2702,7 @@ bool run_scc_dense(ra_program* p, Scc& s)
     }
 
     finish_closure_scc(p, s, ru.out, R, n_stored, total, lv, L, iterations);
-    p->stats.join_candidates += cnt[1];
+    p->stats.join_candidates += visited;
     p->stats.dense_sccs++;
     return true;
 }
@@ -3401,7 +3408,7 @@ void begin_run(ra_program* p)
         for (Relation& r : p->rels) wide_load(p, r);
     }
     p->running = true;
-    p->fixpoint_ms_acc = 0;
+    p->scc_ev_n = 0;
     p->executed_ids = p->rs_skip;
     if (p->cp_every) mkdir(p->cp_dir.c_str(), S_IRWXU | S_IRWXG | S_IROTH | S_IXOTH);
 }
@@ -3442,7 +3449,12 @@ void finish_run(ra_program* p)
     }
     p->phase_events.clear();
     p->stats.dedup_ms = dms;
-    p->stats.fixpoint_ms = p->fixpoint_ms_acc;
+    for (size_t i = 0; i < p->scc_ev_n; i++) {
+        float ms = 0;
+        cudaEventElapsedTime(&ms, p->scc_ev[i].first, p->scc_ev[i].second);
+        p->stats.fixpoint_ms += ms;
+    }
+    p->scc_ev_n = 0;
     p->stats.value_bits = (uint32_t)p->bits;
     p->executed = true;
     p->running = false;
@@ -3462,14 +3474,19 @@ int step(ra_program* p)
         finish_run(p);
         return -1;
     }
-    CK(cudaEventRecord(p->ev0, p->stream));
+    // the SCC's device time is read when the run ends, after its synchronisation
+    if (p->scc_ev_n == p->scc_ev.size()) {
+        cudaEvent_t a = nullptr, b = nullptr;
+        CK(cudaEventCreate(&a));
+        p->scc_ev.push_back({a, nullptr});
+        CK(cudaEventCreate(&b));
+        p->scc_ev.back().second = b;
+    }
+    const auto ev = p->scc_ev[p->scc_ev_n++];
+    CK(cudaEventRecord(ev.first, p->stream));
     run_scc(p, p->sccs[next]);
     p->sccs[next].done = true;
-    CK(cudaEventRecord(p->ev1, p->stream));
-    CK(cudaEventSynchronize(p->ev1));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, p->ev0, p->ev1);
-    p->fixpoint_ms_acc += ms;
+    CK(cudaEventRecord(ev.second, p->stream));
     // the run ends at the next step, so that counts read after the last SCC are, as
     // the reference prints them there, from before its final delta -> full merge
     return p->sccs[next].id;
@@ -3527,8 +3544,6 @@ int ra_program_create(int device, ra_program** out)
         dev_alloc(p, &p->dscalar, 8);
         dev_alloc(p, &p->derr, 4);
         CK(cudaMallocHost(&p->hscalar, 64));
-        CK(cudaEventCreate(&p->ev0));
-        CK(cudaEventCreate(&p->ev1));
         dev_alloc(p, &p->ctl, 1);
         CK(cudaMallocHost(&p->hctl, sizeof(IterCtl)));
         if (const char* e = getenv("RA_NO_GRAPH")) p->use_graphs = atoi(e) == 0;
@@ -3605,8 +3620,10 @@ int ra_program_destroy(ra_program* p)
     if (p->wide_ev) cudaEventDestroy(p->wide_ev);
     if (p->hscalar) cudaFreeHost(p->hscalar);
     if (p->hctl) cudaFreeHost(p->hctl);
-    if (p->ev0) cudaEventDestroy(p->ev0);
-    if (p->ev1) cudaEventDestroy(p->ev1);
+    for (auto& e : p->scc_ev) {
+        if (e.first) cudaEventDestroy(e.first);
+        if (e.second) cudaEventDestroy(e.second);
+    }
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
     g_ring.remove();
@@ -4086,10 +4103,12 @@ int ra_relation_instance_summary(ra_program* p, int rel, uint64_t* counts, uint6
                                                                            p->n_inst, acc, acc + m);
             LAUNCHED();
         }
-        CK(cudaMemcpyAsync(counts, acc, m * 8, cudaMemcpyDeviceToHost, p->stream));
-        CK(cudaMemcpyAsync(digests, acc + m, m * 8, cudaMemcpyDeviceToHost, p->stream));
-        CK(cudaStreamSynchronize(p->stream));
+        u64* got = host_words(p, 2 * m);
+        CK(cudaMemcpyAsync(got, acc, 2 * m * 8, cudaMemcpyDeviceToHost, p->stream));
         dev_free(p, &acc);
+        CK(cudaStreamSynchronize(p->stream));
+        std::memcpy(counts, got, m * 8);
+        std::memcpy(digests, got + m, m * 8);
     });
 }
 

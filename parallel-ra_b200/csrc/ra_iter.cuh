@@ -76,6 +76,7 @@ struct IterCtl {
     u64 bit_cand[kMaxSccRules];
     u32 bit_exit[kMaxSccRules];
     u64 bit_filter;
+    u64 last_delta, last_full, last_time;   // the latest history entry and iteration end time
     u32 bar_count;                  // blocks arrived at the running barrier
     u32 bar_gen;                    // barrier generation (bumped on release)
     u32 bar_flags;                  // flags / done / heavy_n as the last arriver saw them
@@ -958,15 +959,16 @@ __device__ void end_of_iteration(IterCtl* __restrict__ ctl, const SccPlan& plan,
         ctl->candidates += cands;
         ctl->new_tuples += added;
         ctl->bit_filter = 4 * added < 3 * cands;
-        if (ctl->iteration < ctl->time_cap) history[2 * plan.hist_cap + ctl->iteration] = global_ns();
+        ctl->last_time = global_ns();
+        if (ctl->iteration < ctl->time_cap) history[2 * plan.hist_cap + ctl->iteration] = ctl->last_time;
         ctl->iteration++;
         ctl->epoch++;
         ctl->batch_pos++;
         cont = true;
         if (records) {
             ctl->batch_pos = 0;
-            history[2 * ctl->hist_n] = sum_delta;
-            history[2 * ctl->hist_n + 1] = sum_full;
+            history[2 * ctl->hist_n] = ctl->last_delta = sum_delta;
+            history[2 * ctl->hist_n + 1] = ctl->last_full = sum_full;
             ctl->hist_n++;
             cont = plan.fixpoint && sum_delta != 0;
         }
