@@ -302,7 +302,7 @@ class Program:
         """Full relation rows (data columns + id) in lexicographic order."""
         n = self.full_count(rel)
         w = self._arity[rel] + 1
-        buf = np.zeros((max(n, 1), w), dtype=np.uint64)
+        buf = np.empty((max(n, 1), w), dtype=np.uint64)   # every row is written
         got = C.c_uint64()
         self._ck(self._L.ra_relation_dump_full(self._p, rel, _u64(buf), n, C.byref(got)), "dump_full")
         return buf[:got.value]
