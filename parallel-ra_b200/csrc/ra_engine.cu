@@ -198,9 +198,10 @@ struct ra_program {
     u64* dscalar = nullptr;       // device scalars: [0] total, [1] max, [2] flag
     u64* hscalar = nullptr;       // pinned host mirror
     u32* derr = nullptr;
-    u32* hist_buf = nullptr;
-    u64* hist_off = nullptr;
-    u64 hist_cap = 0;
+    u64* sort_counts = nullptr;   // radix_sort: digit counts of 8 passes, their tile counters
+    u64* sort_status = nullptr;   // look-back words, tagged by pass
+    u64 sort_status_cap = 0;
+    u32 sort_tag = 0;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> dedup_events;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> phase_events;
     // device-driven SCC runs (graph mode)
@@ -518,34 +519,44 @@ void radix_sort(ra_program* p, u64* k, u64* v, u64 n, int lo, int hi)
 {
     if (n <= 1 || hi <= lo) return;
     ensure_tmp(p, n);
-    int g = grid_for(n);
-    if (g > 4 * kSms) g = 4 * kSms;
-    u64 chunk = (n + g - 1) / g;
-    g = (int)((n + chunk - 1) / chunk);
-    u64 hn = (u64)kRadix * g;
-    if (hn > p->hist_cap) {
-        dev_free(p, &p->hist_buf);
-        dev_free(p, &p->hist_off);
-        dev_alloc(p, &p->hist_buf, hn);
-        dev_alloc(p, &p->hist_off, hn);
-        p->hist_cap = hn;
+    const int passes = (hi - lo + kRadixBits - 1) / kRadixBits;   // at most 8
+    const u64 tiles = (n + kSortTile - 1) / kSortTile;
+    if (tiles * kRadix > p->sort_status_cap || p->sort_tag + passes >= (1u << 24)) {
+        if (tiles * kRadix > p->sort_status_cap) {
+            dev_free(p, &p->sort_status);
+            p->sort_status_cap = 0;
+            dev_alloc(p, &p->sort_status, tiles * kRadix * 3 / 2);
+            p->sort_status_cap = tiles * kRadix * 3 / 2;
+        }
+        CK(cudaMemsetAsync(p->sort_status, 0, p->sort_status_cap * 8, p->stream));
+        p->sort_tag = 0;
     }
+    if (!p->sort_counts) dev_alloc(p, &p->sort_counts, 8 * kRadix + 8);
+    CK(cudaMemsetAsync(p->sort_counts, 0, (8 * kRadix + 8) * 8, p->stream));
+    sort_counts_kernel<<<(int)std::min<u64>((n + 4 * kThreads - 1) / (4 * kThreads), kSms * 4), kThreads, 0, p->stream>>>(
+        k, n, lo, passes, p->sort_counts);
+    LAUNCHED();
     u64 *sk = k, *sv = v, *dk = p->tk, *dv = p->tv;
-    int passes = 0;
-    for (int shift = lo; shift < hi; shift += kRadixBits) {
-        radix_histogram<<<g, kThreads, 0, p->stream>>>(sk, n, chunk, shift, p->hist_buf, g);
-        LAUNCHED();
-        scan_exclusive<u32>(p, p->hist_buf, hn, p->hist_off, false);
-        radix_scatter<<<g, kThreads, 0, p->stream>>>(sk, sv, dk, dv, n, chunk, shift, p->hist_off, g);
+    for (int ps = 0; ps < passes; ps++) {
+        sort_array_kernel<<<(int)std::min<u64>(tiles, kSms * 3), kThreads, 0, p->stream>>>(
+            sk, sv, dk, dv, n, lo + ps * kRadixBits, p->sort_counts + ps * kRadix,
+            (u32*)(p->sort_counts + 8 * kRadix + ps), p->sort_status, ++p->sort_tag, p->hscalar + 7);
         LAUNCHED();
         std::swap(sk, dk);
         std::swap(sv, dv);
-        passes++;
     }
     if (passes & 1) {
         CK(cudaMemcpyAsync(k, sk, n * 8, cudaMemcpyDeviceToDevice, p->stream));
         CK(cudaMemcpyAsync(v, sv, n * 8, cudaMemcpyDeviceToDevice, p->stream));
     }
+}
+
+// After a synchronisation: did a look-back of an array's sort give up?
+void check_sorts(ra_program* p)
+{
+    if (!p->hscalar[7]) return;
+    p->hscalar[7] = 0;
+    fail(p, RA_E_TIMEOUT, "a device-side look-back wait of a sort gave up");
 }
 
 int key_bits(ra_program* p, const Relation& r) { return (int)r.arity * p->bits; }
@@ -3343,9 +3354,9 @@ void release_buffers(ra_program* p)
     dev_free(p, &p->nids);
     dev_free(p, &p->tk);
     dev_free(p, &p->tv);
-    dev_free(p, &p->hist_buf);
-    dev_free(p, &p->hist_off);
-    p->cand_cap = p->rank_cap = p->cnt_cap = p->n_cap = p->t_cap = p->hist_cap = 0;
+    dev_free(p, &p->sort_counts);
+    dev_free(p, &p->sort_status);
+    p->cand_cap = p->rank_cap = p->cnt_cap = p->n_cap = p->t_cap = p->sort_status_cap = 0;
     dev_free(p, &p->dcand);
     dev_free(p, &p->dloser);
     p->dcand_cap = 0;
@@ -3431,6 +3442,7 @@ void finish_run(ra_program* p)
 {
     merge_pending(p);
     CK(cudaStreamSynchronize(p->stream));
+    check_sorts(p);
     double dms = 0;
     for (auto& e : p->dedup_events) {
         float m = 0;
@@ -3544,6 +3556,7 @@ int ra_program_create(int device, ra_program** out)
         dev_alloc(p, &p->dscalar, 8);
         dev_alloc(p, &p->derr, 4);
         CK(cudaMallocHost(&p->hscalar, 64));
+        p->hscalar[7] = 0;   // set by a sort whose look-back gave up
         dev_alloc(p, &p->ctl, 1);
         CK(cudaMallocHost(&p->hctl, sizeof(IterCtl)));
         if (const char* e = getenv("RA_NO_GRAPH")) p->use_graphs = atoi(e) == 0;
@@ -3584,8 +3597,8 @@ int ra_program_destroy(ra_program* p)
     dev_free(p, &p->sums);
     dev_free(p, &p->dscalar);
     dev_free(p, &p->derr);
-    dev_free(p, &p->hist_buf);
-    dev_free(p, &p->hist_off);
+    dev_free(p, &p->sort_counts);
+    dev_free(p, &p->sort_status);
     dev_free(p, &p->ctl);
     dev_free(p, &p->dcand);
     dev_free(p, &p->dloser);
@@ -4157,6 +4170,7 @@ int ra_relation_dump_full(ra_program* p, int rel, uint64_t* host_rows, uint64_t 
             ~Free() { dev_free(p, q); }
         } free_rows{p, &rows};
         rows_to_host(p, host_rows, rows, m * (r.arity + 1) * 8);
+        check_sorts(p);
     });
 }
 
