@@ -2845,7 +2845,7 @@ bool run_scc_sparse(ra_program* p, Scc& s)
             CK(cudaMemcpyAsync(hc.data(), B.ctr, 4 * 8, cudaMemcpyDeviceToHost, p->stream));
             CK(cudaMemcpyAsync(total.data(), a.level_total, kSpLevels * 8, cudaMemcpyDeviceToHost, p->stream));
             CK(cudaStreamSynchronize(p->stream));
-            if (fl & ~kSpArena) return false;
+            if ((fl & ~kSpArena) || hc[1] >> 32) return false;   // positions within a level are 32 bits
             if (!(fl & kSpArena)) break;
             if (round) return false;
             a.arena_cap = std::max(a.arena_cap, hc[1]);   // the whole search's needs are known
