@@ -202,11 +202,11 @@ def dense_roofline(d, peak, peak_kind):
             "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
             "bytes_model": "16 B written per new tuple (key + id)",
             "share_of_dense_time": d["emit_ms"] / tot if tot else None,
-            "dense_search": {"kernels": "dense_closure_kernel / dense_closure_warp_kernel", "ms": d["search_ms"],
+            "dense_search": {"kernels": "dense_ms_kernel (dense_closure_kernel above 18,944 values)", "ms": d["search_ms"],
                              "share_of_dense_time": d["search_ms"] / tot if tot else None,
                              "edges_per_s": d["candidates"] / (d["search_ms"] / 1e3) if d["search_ms"] else None,
-                             "bound": "SM issue: shared-memory bit sets and atomics, adjacency L2-resident "
-                                      "(ncu: sm__throughput ~73%, DRAM idle)"}}
+                             "bound": "SM issue and shared-memory conflicts in wide levels, one L2 round trip and two "
+                                      "barriers in narrow ones; adjacency L2-resident, DRAM idle"}}
 
 
 def reduce_ranks(total_ms, count, device):
@@ -469,22 +469,32 @@ def run_ours(args, rank, world, local_rank):
     peak, peak_kind = load_peaks()
     achieved = (dedup_bytes / dedup_launches) / ((dedup_ms / dedup_launches) / 1e3) / 1e9 if dedup_launches else 0.0
     bitmap = st.bitmap_relations > 0
-    roofline = dense_roofline(dense, peak, peak_kind) if dense["sccs"] else {"kernel": "join_fused_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roofline = dense_roofline(dense, peak, peak_kind) if dense["sccs"] else {"kernel": "join_bitmap_kernel" if bitmap else "join_fused_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": peak_kind,
                 "traffic": None if bitmap else TRAFFIC_PER_ALGO_BYTE * dedup_bytes / max(dedup_launches, 1),
                 "traffic_note": ("not captured for the bitmap path" if bitmap else
                                  "ncu DRAM read+write per launch, measured on tc-er20 and scaled by units processed"),
                 "launches": int(dedup_launches), "avg_launch_us": 1e3 * dedup_ms / max(dedup_launches, 1),
                 "bytes_per_launch": dedup_bytes / max(dedup_launches, 1),
-                "bytes_model": ("8 B per candidate (the inner key; the claim is a bit test and an atomicOr on a "
-                                "bitmap word, mostly L2-resident) + 24 B per outer delta row" if bitmap else
+                "bytes_model": ("8 B per candidate (the inner key; the claim is one reduction into a bitmap "
+                                "word, mostly L2-resident) + 24 B per outer delta row" if bitmap else
                                 "48 B per candidate (8 B inner key read, 8 B candidate write, 16 B seen-slot read "
                                 "+ 16 B write) + 24 B per outer delta row (key, row offset, CSR start)")}
+    if prog_kind == "tc" and not dense["sccs"] and not bitmap and st.dedup_launches < st.iterations:
+        # the timed steps ran the sparse row closure; the instrumented pass keeps the iteration loop
+        # (per-launch events), whose join roofline is kept beside it
+        moved = 24.0 * st.new_tuples
+        roofline = {"kernel": "sparse_search_kernel + sparse_place_kernel", "bound": "L2 round trips (search), DRAM "
+                    "writes scattered over the levels (placement)", "achieved": moved / (st.fixpoint_ms / 1e3) / 1e9,
+                    "peak": peak, "unit": "GB/s", "frac": moved / (st.fixpoint_ms / 1e3) / 1e9 / peak,
+                    "peak_kind": peak_kind, "traffic": None,
+                    "bytes_model": "24 B per new tuple (16 B log row written, 4 B search order written and read) over "
+                                   "the device time of the program's SCCs", "loop": roofline}
     if not dense["sccs"] and not bitmap and dedup_launches and world == 1:
         # the claims' own ceiling on this GPU: random 16-byte CAS on a table of the seen set's size
         cal = P.engine.calibrate_random_access(dev, slots=max(1 << 20, int(tc / 0.45)), ops=64 << 20)
         claims_per_s = st.join_candidates / (dedup_ms / max(1, min(args.steps, 3)) / 1e3) if dedup_ms else 0.0
-        roofline["random_access_ceiling"] = {
+        roofline.get("loop", roofline)["random_access_ceiling"] = {
             "cas16_per_s": cal["cas16_per_s"], "load8_per_s": cal["load8_per_s"], "table_bytes": cal["table_bytes"],
             "claims_per_s": claims_per_s, "claims_frac_of_cas16": claims_per_s / cal["cas16_per_s"],
             "note": "every candidate claims one 16-byte slot of a table far larger than L2; this GPU's rate "
