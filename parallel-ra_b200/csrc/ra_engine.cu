@@ -1521,6 +1521,7 @@ int launch_iteration(ra_program* p, DevScc& d, cudaGraphConditionalHandle cond, 
         a.dst_keys = ref ? p->stage_k[r.out_slot] : out.keys;
         a.dst_ids = ref ? p->stage_v[r.out_slot] : out.ids;
         a.passes = ref ? d.passes[r.out_slot] : 0;
+        a.last_shift = std::max(0, key_bits(p, out) - kRadixBits);
         a.stage_cap = p->stage_cap;
         if (tail) {
             a.tail_on = 1;
@@ -1548,7 +1549,14 @@ int launch_iteration(ra_program* p, DevScc& d, cudaGraphConditionalHandle cond, 
                 SortPassArgs a{};
                 a.rel = sl;
                 a.pass = ps;
-                a.shift = ps * kRadixBits;
+                // the last digit is the key's top 8 bits, whatever the digits before it leave
+                a.last_pass = P - 1;
+                a.last_shift = std::max(0, key_bits(p, r) - kRadixBits);
+                a.shift = std::min(ps * kRadixBits, a.last_shift);
+                // two launches save one or more only from three digits on
+                a.buckets = P > 2;
+                a.log_k = r.keys;
+                a.log_v = r.ids;
                 a.src_k = ps == 0 ? p->stage_k[sl] : p->sort_k[(ps - 1) & 1];
                 a.src_v = ps == 0 ? p->stage_v[sl] : p->sort_v[(ps - 1) & 1];
                 a.dst_log = (ps == P - 1) ? 1 : 0;
@@ -2371,7 +2379,7 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
     p->stats.dedup_launches += (u64)d.rules.size() * h.iteration;
     // algorithmic bytes: a hash seen set costs 48 B per candidate (inner key read, candidate
     // write, 16-byte slot read + write); a bitmap one 8 B (the inner key; the claim is a bit
-    // test and an atomicOr on a mostly L2-resident word); 24 B per outer row either way
+    // reduction into a mostly L2-resident word); 24 B per outer row either way
     bool bitmap_scc = false;
     for (int sl = 0; sl < d.plan.n_rels; sl++) bitmap_scc = bitmap_scc || d.bit[sl].seen;
     p->stats.dedup_bytes += (bitmap_scc ? 8 : 48) * h.candidates + 24 * h.outer_rows;

@@ -19,8 +19,11 @@
 //                  straight into the relation's log, intern ids; the last tile
 //                  of the last rule runs the iteration end: region bump,
 //                  history, intern counters, graph condition
-//   (reference id order only) digit histograms in select, onesweep LSD radix
-//   passes over the new delta, then a separate iteration-end launch
+//   join_bitmap, bitmap_select  the same two steps for output relations whose seen
+//                  set is a bitmap: a claim is one reduction, the log follows the rows
+//   (reference id order only) digit histograms in select, radix launches over the
+//   new delta (by buckets of the top digit, or onesweep LSD passes), then a separate
+//   iteration-end launch
 // An iteration that finds a buffer too small stops before select writes
 // anything; claims made so far are idempotent, so the host grows the buffer
 // and replays the same iteration (same epoch, same stream positions).
@@ -1042,6 +1045,7 @@ struct SelectArgs {
     u64* dst_ids;
     int to_log;
     int passes;               // digit histograms to accumulate (reference ids)
+    int last_shift;           // shift of the last of them
     u64 stage_cap;
     // a slice of the rule's outer rows: candidates at buffer index 0; `appended` winners of
     // this iteration already in the relation's log (earlier rules and slices), `id_appended`
@@ -1221,7 +1225,7 @@ __global__ void __launch_bounds__(kThreads, RA_SELECT_MIN_BLOCKS) select_kernel(
                 dk[dst_off + r] = kk;
                 dv[dst_off + r] = tag_word | (id_ctr + r);
                 for (int ps = 0; ps < a.passes; ps++)
-                    atomicAdd(&s_hist[ps][(kk >> (ps * kRadixBits)) & (kRadix - 1)], 1u);
+                    atomicAdd(&s_hist[ps][(kk >> min(ps * kRadixBits, a.last_shift)) & (kRadix - 1)], 1u);
             }
             if (a.inst_base) {
                 u64* row = a.inst_new + ctl->iteration * a.n_inst;
@@ -1256,7 +1260,7 @@ __global__ void __launch_bounds__(kThreads, RA_SELECT_MIN_BLOCKS) select_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// onesweep LSD radix pass over a relation's staged rows
+// radix launches over a relation's staged rows
 // ---------------------------------------------------------------------------
 constexpr int kSortIpt = 8;
 constexpr int kSortTile = kThreads * kSortIpt;
@@ -1443,7 +1447,11 @@ struct SortPassArgs {
     u64* dst_k;               // when dst_log: the log base (rows go to base + full_n + delta_n)
     u64* dst_v;
     int dst_log;
-    u64 log_cap;              // rows the relation's log holds (dst_log)
+    u64 log_cap;              // rows the relation's log holds
+    int buckets;              // the relation sorts in two launches when sort_fits
+    int last_pass, last_shift;   // the top digit's pass and shift
+    u64* log_k;               // the log base, for the second of those launches
+    u64* log_v;
     int n_rules_in;           // rules writing this relation
     int rules_in[kMaxSccRules];
 };
@@ -1462,6 +1470,57 @@ struct SortSmem {
     u64 sm[kWarps + 1];
     u32 tile;
 };
+
+// Ranks the tn rows held by the block (kk, thread order of sort_tiles) by digit: rk[r] counts the
+// row's equals before it in its warp, S.loc[d] is digit d's first place and S.wcnt[w][d] the
+// warp's share before it.  S.wcnt is zero and synchronised on entry.  Returns the count of
+// digit threadIdx.x.
+__device__ __forceinline__ u32 sort_rank(SortSmem& S, const u64 (&kk)[kSortIpt], u32 (&rk)[kSortIpt], u32 tn, int shift)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int r = 0; r < kSortIpt; r++) {
+        const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
+        const bool valid = li < tn;
+        const int d = valid ? (int)((kk[r] >> shift) & (kRadix - 1)) : (kRadix + lane);
+        const u32 peers = __match_any_sync(0xffffffffu, d);
+        const u32 before = __popc(peers & lanemask_lt());
+        const u32 prior = valid ? S.wcnt[warp][d] : 0;
+        __syncwarp();
+        if (valid && before == 0) S.wcnt[warp][d] = prior + __popc(peers);
+        __syncwarp();
+        rk[r] = prior + before;
+    }
+    __syncthreads();
+    // digit totals of the tile -> tile-local run starts; per-warp bases inside each run
+    const int d = threadIdx.x;   // kThreads == kRadix
+    u32 run = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const u32 c = S.wcnt[w][d];
+        S.wcnt[w][d] = run;
+        run += c;
+    }
+    u64 tot;
+    S.loc[d] = (u32)block_exclusive_scan((u64)run, S.sm, &tot);
+    return run;
+}
+
+// Places the ranked rows in shared memory in digit order (stable).  S.loc and S.wcnt synchronised.
+__device__ __forceinline__ void sort_put(SortSmem& S, const u64 (&kk)[kSortIpt], const u64 (&vv)[kSortIpt],
+                                         const u32 (&rk)[kSortIpt], u32 tn, int shift)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int r = 0; r < kSortIpt; r++) {
+        const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
+        if (li >= tn) continue;
+        const int dd = (int)((kk[r] >> shift) & (kRadix - 1));
+        const u32 pos = S.loc[dd] + S.wcnt[warp][dd] + rk[r];
+        S.k[pos] = kk[r];
+        S.v[pos] = vv[r];
+    }
+}
 
 template <typename Timeout>
 __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ src_k, const u64* __restrict__ src_v,
@@ -1492,33 +1551,8 @@ __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ 
             kk[r] = li < tn ? src_k[t0 + li] : 0;
             vv[r] = li < tn ? src_v[t0 + li] : 0;
         }
-#pragma unroll
-        for (int r = 0; r < kSortIpt; r++) {
-            const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
-            const bool valid = li < tn;
-            const int d = valid ? (int)((kk[r] >> shift) & (kRadix - 1)) : (kRadix + lane);
-            const u32 peers = __match_any_sync(0xffffffffu, d);
-            const u32 before = __popc(peers & lanemask_lt());
-            const u32 prior = valid ? S.wcnt[warp][d] : 0;
-            __syncwarp();
-            if (valid && before == 0) S.wcnt[warp][d] = prior + __popc(peers);
-            __syncwarp();
-            rk[r] = prior + before;
-        }
-        __syncthreads();
-        // digit totals of the tile -> tile-local run starts; per-warp bases inside each run
         const int d = threadIdx.x;   // kThreads == kRadix
-        u32 run = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-            const u32 c = S.wcnt[w][d];
-            S.wcnt[w][d] = run;
-            run += c;
-        }
-        {
-            u64 tot;
-            S.loc[d] = (u32)block_exclusive_scan((u64)run, S.sm, &tot);
-        }
+        const u32 run = sort_rank(S, kk, rk, tn, shift);
         // look-back for this digit across tiles (one thread per digit)
         u64* st = status + tile * kRadix + d;
         u64 excl = 0;
@@ -1545,16 +1579,7 @@ __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ 
         }
         S.out[d] = S.gstart[d] + excl;
         __syncthreads();
-        // place the tile in shared memory in digit order (stable)
-#pragma unroll
-        for (int r = 0; r < kSortIpt; r++) {
-            const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
-            if (li >= tn) continue;
-            const int dd = (int)((kk[r] >> shift) & (kRadix - 1));
-            const u32 pos = S.loc[dd] + S.wcnt[warp][dd] + rk[r];
-            S.k[pos] = kk[r];
-            S.v[pos] = vv[r];
-        }
+        sort_put(S, kk, vv, rk, tn, shift);
         __syncthreads();
         // each digit's run is contiguous in the output: coalesced writes
         for (u32 q = threadIdx.x; q < tn; q += kThreads) {
@@ -1568,16 +1593,107 @@ __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict__ ctl, SortPassArgs a,
+// The rows of the top digits' buckets (from `src`, bucket after bucket) to dk / dv in key order: a
+// block per bucket, by comparing each row with all others (up to kSortCompare rows: one pass, a
+// few compares per row and cycle) or digit by digit in shared memory.
+constexpr u32 kSortCompare = 512;
+__device__ __forceinline__ void sort_buckets(SortSmem& S, const u64* __restrict__ src_k, const u64* __restrict__ src_v,
+                                             u64* __restrict__ dk, u64* __restrict__ dv, u32 count, int top_shift)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 tot;
+    S.gstart[threadIdx.x] = block_exclusive_scan((u64)count, S.sm, &tot);
+    S.out[threadIdx.x] = count;
+    __syncthreads();
+    for (int b = blockIdx.x; b < kRadix; b += gridDim.x) {
+        const u32 tn = (u32)S.out[b];   // at most kSortTile (sort_fits)
+        const u64 at = S.gstart[b];
+        if (tn == 0) continue;
+        if (tn <= kSortCompare) {
+            constexpr int kOwn = kSortCompare / kThreads;
+            u64 k[kOwn], v[kOwn];
+            u32 less[kOwn];
+#pragma unroll
+            for (int e = 0; e < kOwn; e++) {
+                const u32 i = threadIdx.x + e * kThreads;
+                k[e] = i < tn ? src_k[at + i] : ~0ull;
+                v[e] = i < tn ? src_v[at + i] : 0;
+                S.k[i] = k[e];
+                less[e] = 0;
+            }
+            __syncthreads();
+            if (warp * 32 < tn)
+                for (u32 j = 0; j < tn; j++) {
+                    const u64 o = S.k[j];
+#pragma unroll
+                    for (int e = 0; e < kOwn; e++)
+                        less[e] += o < k[e] || (o == k[e] && j < threadIdx.x + e * kThreads);
+                }
+#pragma unroll
+            for (int e = 0; e < kOwn; e++)
+                if (threadIdx.x + e * kThreads < tn) {
+                    dk[at + less[e]] = k[e];
+                    dv[at + less[e]] = v[e];
+                }
+        } else {
+            u64 kk[kSortIpt], vv[kSortIpt];
+            u32 rk[kSortIpt];
+            for (int shift = 0; shift < top_shift; shift += kRadixBits) {
+#pragma unroll
+                for (int r = 0; r < kSortIpt; r++) {
+                    const u32 li = (u32)(warp * 32 * kSortIpt + r * 32 + lane);
+                    kk[r] = li < tn ? (shift ? S.k[li] : src_k[at + li]) : 0;
+                    vv[r] = li < tn ? (shift ? S.v[li] : src_v[at + li]) : 0;
+                }
+                for (int i = threadIdx.x; i < kWarps * kRadix; i += kThreads) (&S.wcnt[0][0])[i] = 0;
+                __syncthreads();
+                sort_rank(S, kk, rk, tn, shift);
+                __syncthreads();
+                sort_put(S, kk, vv, rk, tn, shift);
+                __syncthreads();
+            }
+            for (u32 q = threadIdx.x; q < tn; q += kThreads) {
+                dk[at + q] = S.k[q];
+                dv[at + q] = S.v[q];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// One launch of a new delta's sort (reference id order).  By digits, lowest first, a launch per
+// digit; when no top digit has more than kSortTile rows, the first launch instead parts the rows
+// by their top digit, the second sorts every bucket in shared memory into the log, and the others
+// return at once.  Bound by each launch's chain of round trips (a few thousand to a hundred
+// thousand rows).  Transitive closure of 100,003 values and 95,000 edges, 78 deltas of 34-bit keys:
+// 5.89 -> 4.11 ms for the fixed point against five digit launches each.
+__global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict__ ctl,
+                                                             const __grid_constant__ SortPassArgs a,
                                                              u64* __restrict__ status, int tile_slot)
 {
     __shared__ SortSmem S;
+    const u32 top = a.buckets ? (u32)min(ctl->sort_hist[a.rel][a.last_pass][threadIdx.x], (u64)kSortTile + 1) : 0u;
     if (ctl->flags) return;
     u64 n = 0;
     for (int q = 0; q < a.n_rules_in; q++) n += ctl->win_n[a.rules_in[q]];
-    if (n == 0 || blockIdx.x >= (n + kSortTile - 1) / kSortTile) return;
+    if (n == 0) return;
+    const u64 ntiles = (n + kSortTile - 1) / kSortTile;
+    if (blockIdx.x >= max(ntiles, (u64)(a.buckets && a.pass == 1 ? kRadix : 0))) return;
     u64* dk = a.dst_k;
     u64* dv = a.dst_v;
+    const bool fits = a.buckets && !__syncthreads_or(top > kSortTile);
+    if (fits && a.pass > 1) return;
+    if (fits && a.pass == 1) {
+        const u64 o = ctl->full_n[a.rel] + ctl->delta_n[a.rel];
+        if (o + n > a.log_cap) {   // as below
+            if (threadIdx.x == 0) atomicOr(&ctl->flags, kFlagOverflow);
+            return;
+        }
+        sort_buckets(S, a.src_k, a.src_v, a.log_k + o, a.log_v + o, top, a.last_shift);
+        return;
+    }
+    if (blockIdx.x >= ntiles) return;
+    const int pass = fits ? a.last_pass : a.pass;
     if (a.dst_log) {
         const u64 o = ctl->full_n[a.rel] + ctl->delta_n[a.rel];
         if (o + n > a.log_cap) {   // select checks this first; never write past the log
@@ -1587,7 +1703,8 @@ __global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict
         dk += o;
         dv += o;
     }
-    sort_tiles(S, a.src_k, a.src_v, dk, dv, n, a.shift, ctl->sort_hist[a.rel][a.pass], tile_counter(ctl, tile_slot),
+    sort_tiles(S, a.src_k, a.src_v, dk, dv, n, fits ? a.last_shift : a.shift, ctl->sort_hist[a.rel][pass],
+               tile_counter(ctl, tile_slot),
                status, iter_tag(ctl, tile_slot), [&] { atomicOr(&ctl->flags, kFlagTimeout); });
 }
 
