@@ -137,8 +137,11 @@ typedef struct ra_stats {
  *                       whose one rule has the transitive-closure shape
  *                       R(z,x) :- R_delta(y,x), S_full(y,z) over values (per
  *                       instance) below 65,536 runs as one breadth-first search
- *                       per row of R in shared memory instead of the hash-set
- *                       path (emission id order, batch size 1). */
+ *                       per row of R in shared memory (32 rows at a time up to
+ *                       18,944 values) instead of the hash-set path (emission
+ *                       id order, batch size 1); 0 also switches off the sparse
+ *                       row-closure evaluator, which runs such SCCs over more
+ *                       values. */
 typedef struct ra_tuning {
     double seen_load_max;
     double seen_grow;

@@ -10,9 +10,10 @@
 // row x's initial delta, and iteration k of the semi-naive loop is level k of
 // all rows' searches.  The evaluator keeps one bit matrix per instance (row x:
 // one bit per value of x's instance) and runs each row's whole search in
-// shared memory -- one CTA per row, bit sets for the known tuples, the
-// frontier and the next level -- adding every level's new-tuple count to the
-// per-iteration (and per-instance) totals.  The result is the same set of
+// shared memory -- a CTA per 32 rows with a bit per row and value (up to kMsMaxN
+// values), or a CTA per row, for the known tuples, the frontier and the next
+// level -- adding every level's new-tuple count to the per-iteration (and
+// per-instance) totals.  The result is the same set of
 // tuples, iteration by iteration, as the hash-set path produces; only the
 // order in which the new tuples enter the log differs (row by row, values
 // ascending).

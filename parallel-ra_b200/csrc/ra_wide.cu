@@ -12,9 +12,8 @@
 //   1. each rule's candidates, in the reference's emission order (outer rows in
 //      trie order, each one's inner matches in trie order; copies in input order),
 //      written into its output relation's candidate buffer after the earlier rules';
-//   2. per output relation: an index sort that puts equal candidates next to each
-//      other in position order; the first of each group wins unless full or delta
-//      holds it;
+//   2. per output relation: a hash table of the candidates that keeps each row's least
+//      position; that candidate wins unless full or delta holds it;
 //   3. ids (tag << 46) | counter assigned to the winners rule by rule in the SCC's
 //      rule order, the counters shared by the relations of one tag, as the
 //      single-rank reference interns them (bucket 0);
@@ -24,8 +23,8 @@
 //
 // An iteration makes two host round trips (candidate counts; winner counts) and
 // runs each phase for all of its small rules or relations in one batched launch
-// (work lists as kernel parameters), so its cost is a few dozen launches
-// however few tuples it moves.
+// (work lists as kernel parameters), and merges full and delta while
+// the host waits, so its cost is some twenty launches however few tuples it moves.
 //
 // (Included inside the engine's anonymous namespace.)
 
