@@ -2881,7 +2881,7 @@ bool run_scc_sparse(ra_program* p, Scc& s)
         sparse_offsets_kernel<<<a.blocks, kThreads, 0, p->stream>>>(a, B.pos);
         LAUNCHED();
         sparse_place_kernel<<<(int)std::min<u64>((a.tiles + kWarps - 1) / kWarps, kSms * 8), kThreads, 0, p->stream>>>(
-            a, B.pos, B.base, R.keys + n_stored, R.ids + n_stored, id0);
+            a, B.pos, B.base, R.keys + n_stored, R.ids + n_stored, sum, id0);
         LAUNCHED();
         CK(cudaStreamSynchronize(p->stream));   // the scratch goes when this returns
     }

@@ -394,11 +394,12 @@ __global__ void __launch_bounds__(kThreads) sparse_offsets_kernel(SparseArgs a, 
 // base[k] + pos + (i - the level's first entry).  Neighbouring tiles write neighbouring runs
 // of each level.  Bound by the chain tile -> level starts -> entries -> stores, so the next
 // tile's start and four entries of a lane are loaded ahead; at sizes beyond L2 by DRAM writes to
-// as many places as there are levels: n = 2^22, 1.07 ms for 1.5 GB; n = 2^18, 20 us (4.6 TB/s).
+// as many places as there are levels, so only the keys go there; ids follow the rows and are
+// written row after row.  n = 2^22, 1.5 GB: 1.06 ms with ids beside their keys, 0.78 so.
 __global__ void __launch_bounds__(kThreads) sparse_place_kernel(SparseArgs a, const u32* __restrict__ pos,
                                                                 const u64* __restrict__ base,
                                                                 u64* __restrict__ keys_out, u64* __restrict__ ids_out,
-                                                                u64 id0)
+                                                                u64 rows, u64 id0)
 {
     constexpr int kAhead = 4;
     const int lane = threadIdx.x & 31;
@@ -435,10 +436,7 @@ __global__ void __launch_bounds__(kThreads) sparse_place_kernel(SparseArgs a, co
                     for (int h = 16; h; h >>= 1)
                         if (__shfl_sync(0xffffffffu, start, l + h) <= j) l += h;
                     const u64 row = __shfl_sync(0xffffffffu, to, l) + (j - __shfl_sync(0xffffffffu, start, l));
-                    if (j < i1) {
-                        keys_out[row] = ((u64)(e[u] & zmask) << a.bits) | (x0 + (e[u] >> a.bits));
-                        ids_out[row] = id0 + row;
-                    }
+                    if (j < i1) keys_out[row] = ((u64)(e[u] & zmask) << a.bits) | (x0 + (e[u] >> a.bits));
                 }
             }
         }
@@ -448,6 +446,7 @@ __global__ void __launch_bounds__(kThreads) sparse_place_kernel(SparseArgs a, co
         at = nlv ? a.tile_at[tile] : 0;
         start = levels[lat + min((u32)lane, nlv)];
     }
+    for (u64 r = (u64)blockIdx.x * kThreads + threadIdx.x; r < rows; r += (u64)gridDim.x * kThreads) ids_out[r] = id0 + r;
 }
 
 }  // namespace ra
