@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kThreads) copy_claim_kernel(IterCtl* __restric
 #pragma unroll
             for (int k = 0; k < kClaimBatch; k++)
                 if (valid[k]) bit_claim(bs, key[k], bits, ctl);
-        } else {
+        } else if (seen) {   // else the candidates are known to be new and different
             claim_batch(seen, seen_cap, key, mine, valid, lm, &ctl->flags);
         }
     }
