@@ -139,7 +139,7 @@ __device__ __forceinline__ void sparse_table_insert(u16* table, u32 key, u32 at)
 // One warp: tiles from the counter, each tile's search to its end.  Bound by the latency of
 // a level's chain -- queue entry (shared memory while the level is narrow) -> edge range ->
 // target, two L2 round trips -- and by its instructions; kSpWarps * kSpCtas warps per SM overlap.
-// Measured on n = 2^22, out-degree 0.95 (76M new tuples): 1.98 ms, where the loop's joins,
+// Measured on n = 2^22, out-degree 0.95 (76M new tuples): 1.94 ms, where the loop's joins,
 // selects and tail kernel take 8.6 ms and clearing its seen set 1.2 ms.  Tiles of 8, 16 and 32 rows
 // with 40 to 48 warps per SM: 3.2, 2.0 and 2.1 ms; 32-bit filter words per warp 512 and 1,024:
 // 2.6 and 2.0 ms (a hit scans the queue, so full filters cost the largest tiles most).
@@ -322,7 +322,14 @@ __global__ void __launch_bounds__(kSpWarps * 32, kSpCtas) sparse_search_kernel(S
             a.tile_lv[tile] = lat;
             a.tile_nlv[tile] = nlv;
         }
-        for (u32 i = lane; i < fresh_n; i += 32) a.arena[at + i] = __ldcg(&q[n0 + i]);
+        for (u32 i0 = lane; i0 < fresh_n; i0 += 128) {   // four entries of a lane in flight
+            u32 e[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = i0 + u * 32 < fresh_n ? __ldcg(&q[n0 + i0 + u * 32]) : 0u;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (i0 + u * 32 < fresh_n) a.arena[at + i0 + u * 32] = e[u];
+        }
         u32* blk = a.block_lv + (u64)(tile >> kSpBlockShift) * kSpLevels;
         for (u32 k = lane; k <= nlv; k += 32) {
             const u32 s = __ldcg(&lv[k]);
