@@ -107,7 +107,8 @@ struct Relation {
     u64 full_n = 0, delta_n = 0;
     bool full_sorted = true;    // full region in trie order (lexicographic on (key, id))
     bool delta_sorted = true;   // delta region in trie order
-    bool keys_unique = true;    // no two stored tuples share data columns
+    bool keys_unique = true;    // no two loaded tuples share data columns
+    bool appended = false;      // restart rows stand after the others, unchecked: any may repeat another
     u64 full_version = 0, delta_version = 0;
     // seen set over data columns
     Slot* seen = nullptr;
@@ -607,6 +608,7 @@ void pack_relation(ra_program* p, Relation& r)
     r.full_n = r.delta_n = r.newt_n = 0;
     r.full_sorted = r.delta_sorted = true;
     r.keys_unique = true;
+    r.appended = false;
     r.full_version = fresh_stamp();
     r.delta_version = fresh_stamp();
     if (r.raw_n == 0) return;
@@ -674,6 +676,7 @@ void restore_loaded(ra_program* p, Relation& r)
     r.full_n = r.delta_n = r.newt_n = 0;
     r.full_sorted = r.delta_sorted = true;
     r.keys_unique = r.l_keys_unique;
+    r.appended = false;
     // same content as when packed: caches built on the loaded state stay valid
     r.full_version = r.l_full_stamp;
     r.delta_version = r.l_delta_stamp;
@@ -1771,6 +1774,7 @@ void load_restart_delta(ra_program* p, Relation& r)
     CK(cudaStreamSynchronize(p->stream));
     dev_free(p, &raw);
     r.delta_n = n;
+    r.appended = true;
     r.delta_sorted = false;
     r.full_sorted = false;
     r.full_version = fresh_stamp();
@@ -2101,13 +2105,14 @@ void launch_persistent(ra_program* p, const DevScc& d)
 // empty, the SCC runs one iteration, and the rule copies distinct rows with every column kept (the
 // copy that starts a transitive closure): its launch then claims nothing and no seen set is cleared
 // (4M rows: the copy 180 -> 24 us, and 100 us of clearing).  A later SCC that needs the table builds it
-// from the rows, at the cost of the claims.
+// from the rows, at the cost of the claims.  A restart's rows are taken as the dump holds them, and
+// again by every SCC that lists their relation, so they may repeat: their copies claim.
 bool distinct_output(ra_program* p, const Scc& s, const DevScc& d, int sl)
 {
     const Relation& out = p->rels[d.rel_of_slot[sl]];
     if (s.fixpoint || p->use_persist || d.rm.n_rules_in[sl] != 1 || out.full_n + out.delta_n) return false;
     const Rule& ru = s.rules[d.rm.rules_in[sl][0]];
-    if (ru.kind == kJoin || !p->rels[ru.in0].keys_unique) return false;
+    if (ru.kind == kJoin || !p->rels[ru.in0].keys_unique || p->rels[ru.in0].appended) return false;
     const Projection& pj = d.rules[d.rm.rules_in[sl][0]].pj;
     u32 kept = 0;
     for (int j = 0; j < pj.n; j++) kept |= 1u << pj.col[j];
