@@ -199,10 +199,11 @@ struct ra_program {
     u64* dscalar = nullptr;       // device scalars: [0] total, [1] max, [2] flag
     u64* hscalar = nullptr;       // pinned host mirror
     u32* derr = nullptr;
-    u64* sort_counts = nullptr;   // radix_sort: digit counts of 8 passes, their tile counters
+    u64* sort_counts = nullptr;   // radix_sort: digit counts of 8 passes, their tile counters, did one give up
     u64* sort_status = nullptr;   // look-back words, tagged by pass
     u64 sort_status_cap = 0;
     u32 sort_tag = 0;
+    u64 sort_polls = kSpinLimit;  // of a look-back; RA_SORT_POLLS=0: every one of an array's sort gives up
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> dedup_events;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> phase_events;
     // device-driven SCC runs (graph mode)
@@ -516,6 +517,10 @@ void ensure_tmp(ra_program* p, u64 n)
     }
 }
 
+constexpr u64 kSortWords = 8 * kRadix + 9;
+
+// (k, v) rows by the bits [lo, hi) of k.  Nothing may use the rows as indices or positions before
+// check_sorts has seen, after a synchronisation, that no look-back gave up.
 void radix_sort(ra_program* p, u64* k, u64* v, u64 n, int lo, int hi)
 {
     if (n <= 1 || hi <= lo) return;
@@ -532,8 +537,8 @@ void radix_sort(ra_program* p, u64* k, u64* v, u64 n, int lo, int hi)
         CK(cudaMemsetAsync(p->sort_status, 0, p->sort_status_cap * 8, p->stream));
         p->sort_tag = 0;
     }
-    if (!p->sort_counts) dev_alloc(p, &p->sort_counts, 8 * kRadix + 8);
-    CK(cudaMemsetAsync(p->sort_counts, 0, (8 * kRadix + 8) * 8, p->stream));
+    if (!p->sort_counts) dev_alloc(p, &p->sort_counts, kSortWords);
+    CK(cudaMemsetAsync(p->sort_counts, 0, kSortWords * 8, p->stream));
     sort_counts_kernel<<<(int)std::min<u64>((n + 4 * kThreads - 1) / (4 * kThreads), kSms * 4), kThreads, 0, p->stream>>>(
         k, n, lo, passes, p->sort_counts);
     LAUNCHED();
@@ -541,7 +546,8 @@ void radix_sort(ra_program* p, u64* k, u64* v, u64 n, int lo, int hi)
     for (int ps = 0; ps < passes; ps++) {
         sort_array_kernel<<<(int)std::min<u64>(tiles, kSms * 3), kThreads, 0, p->stream>>>(
             sk, sv, dk, dv, n, lo + ps * kRadixBits, p->sort_counts + ps * kRadix,
-            (u32*)(p->sort_counts + 8 * kRadix + ps), p->sort_status, ++p->sort_tag, p->hscalar + 7);
+            (u32*)(p->sort_counts + 8 * kRadix + ps), p->sort_status, ++p->sort_tag, p->sort_polls,
+            p->sort_counts + kSortWords - 1, p->hscalar + 7);
         LAUNCHED();
         std::swap(sk, dk);
         std::swap(sv, dv);
@@ -552,17 +558,25 @@ void radix_sort(ra_program* p, u64* k, u64* v, u64 n, int lo, int hi)
     }
 }
 
-// After a synchronisation: did a look-back of an array's sort give up?
-void check_sorts(ra_program* p)
+// After a synchronisation: did a look-back of an array's sort give up?  If so, the rows sorted last
+// are not those they were sorted from; `r` forgets its sorted copy of them.
+void check_sorts(ra_program* p, Relation* r = nullptr)
 {
     if (!p->hscalar[7]) return;
     p->hscalar[7] = 0;
+    if (r) r->v_version = ~0ull;
     fail(p, RA_E_TIMEOUT, "a device-side look-back wait of a sort gave up");
 }
 
 int key_bits(ra_program* p, const Relation& r) { return (int)r.arity * p->bits; }
 
-// sort rows lexicographically by (key, id): by id first when keys may repeat
+void wait_sorts(ra_program* p)
+{
+    CK(cudaStreamSynchronize(p->stream));
+    check_sorts(p);
+}
+
+// sort rows lexicographically by (key, id): by id first when keys may repeat (radix_sort's rule holds)
 void sort_rows(ra_program* p, const Relation& r, u64* k, u64* v, u64 n, bool keys_unique)
 {
     if (!keys_unique) {
@@ -638,6 +652,7 @@ void pack_relation(ra_program* p, Relation& r)
     any_equal_adjacent<<<grid_for(r.raw_n), kThreads, 0, p->stream>>>(r.keys, r.raw_n, (u32*)(p->dscalar + 2));
     LAUNCHED();
     bool dup_keys = read_scalar(p, p->dscalar + 2) != 0;
+    check_sorts(p);
     u64 n = r.raw_n;
     if (dup_keys) {
         r.keys_unique = false;
@@ -650,6 +665,7 @@ void pack_relation(ra_program* p, Relation& r)
         flag_distinct_rows<<<grid_for(n), kThreads, 0, p->stream>>>(r.keys, r.ids, n, p->flag);
         LAUNCHED();
         u64 m = scan_exclusive<u32>(p, p->flag, n, p->rank);
+        check_sorts(p);
         ensure_tmp(p, n);
         compact_flagged<<<grid_for(n), kThreads, 0, p->stream>>>(r.keys, r.ids, p->flag, p->rank, n, p->tk, p->tv);
         LAUNCHED();
@@ -690,12 +706,15 @@ void restore_loaded(ra_program* p, Relation& r)
 
 // (key, id) rows of a relation version.  FULL rows are always returned in trie
 // order (a sorted copy when the region is not sorted); DELTA rows are sorted in
-// place when `sorted` is requested.
-void version_rows(ra_program* p, Relation& r, int ver, const u64** k, const u64** v, u64* n, bool sorted = true)
+// place when `sorted` is requested.  A sort is waited for and checked, unless the caller does so
+// (check = false).
+void version_rows(ra_program* p, Relation& r, int ver, const u64** k, const u64** v, u64* n, bool sorted = true,
+                  bool check = true)
 {
     if (ver == RA_DELTA) {
         if (sorted && !r.delta_sorted && r.delta_n > 1) {
             sort_rows(p, r, r.keys + r.full_n, r.ids + r.full_n, r.delta_n, r.keys_unique);
+            if (check) wait_sorts(p);
             r.delta_version = fresh_stamp();
         }
         if (sorted) r.delta_sorted = true;
@@ -715,6 +734,7 @@ void version_rows(ra_program* p, Relation& r, int ver, const u64** k, const u64*
         CK(cudaMemcpyAsync(r.vkeys, r.keys, r.full_n * 8, cudaMemcpyDeviceToDevice, p->stream));
         CK(cudaMemcpyAsync(r.vids, r.ids, r.full_n * 8, cudaMemcpyDeviceToDevice, p->stream));
         sort_rows(p, r, r.vkeys, r.vids, r.full_n, r.keys_unique);
+        if (check) wait_sorts(p);
         r.v_version = r.full_version;
     }
     *k = r.vkeys;
@@ -895,6 +915,7 @@ void full_to_delta(ra_program* p, Relation& r)
     bool sorted = (r.delta_n == 0 && r.full_sorted) || (r.full_n == 0 && r.delta_sorted);
     if (!sorted && n && p->id_order == RA_IDS_REFERENCE) {
         sort_rows(p, r, r.keys, r.ids, n, r.keys_unique);
+        wait_sorts(p);   // the rows become join keys
         sorted = true;
     }
     r.full_n = 0;
@@ -1072,15 +1093,18 @@ void iterate(ra_program* p, Scc& s)
 
     // 5. sort each relation's newt into trie order; then the semi-naive swap
     //    (RAM::local_insert_in_full -> insert_delta_in_full + local_insert_in_delta)
+    bool sorting = false;
     for (int ri : s.rels) {
         Relation& r = p->rels[ri];
         if (r.newt_n > 1 && p->id_order == RA_IDS_REFERENCE) {
             u64* nk = r.keys + r.full_n + r.delta_n;
             u64* nv = r.ids + r.full_n + r.delta_n;
             radix_sort(p, nk, nv, r.newt_n, 0, key_bits(p, r));
+            sorting = true;
         }
         p->stats.new_tuples += r.newt_n;
     }
+    if (sorting) wait_sorts(p);
     for (int ri : s.rels) {
         Relation& r = p->rels[ri];
         delta_to_full(r);
@@ -1672,6 +1696,7 @@ void dump_region(ra_program* p, Relation& r, const u64* keys, const u64* ids, u6
         dev_free(p, &tk);
         dev_free(p, &tv);
         dev_free(p, &rows);
+        check_sorts(p);
     }
     write_rows_file(p, r, host, n, path);
 }
@@ -3478,7 +3503,6 @@ void finish_run(ra_program* p)
 {
     merge_pending(p);
     CK(cudaStreamSynchronize(p->stream));
-    check_sorts(p);
     double dms = 0;
     for (auto& e : p->dedup_events) {
         float m = 0;
@@ -3600,6 +3624,7 @@ int ra_program_create(int device, ra_program** out)
         if (const char* e = getenv("RA_PERSIST")) p->use_persist = atoi(e) != 0;
         if (const char* e = getenv("RA_REACH")) p->use_reach = atoi(e) != 0;
         if (const char* e = getenv("RA_KERNEL_EVENTS")) p->kernel_events = atoi(e) != 0;
+        if (const char* e = getenv("RA_SORT_POLLS")) p->sort_polls = std::min<u64>(strtoull(e, nullptr, 10), kSpinLimit);
     });
     if (st != RA_OK) {
         delete p;
@@ -3891,6 +3916,7 @@ static int end_failed_run(ra_program* p, int st)
         if (g) cudaGraphDestroy(g);
     }
     if (p->stream) cudaStreamSynchronize(p->stream);
+    p->hscalar[7] = 0;    // a sort that gave up, too
     cudaGetLastError();   // clear a non-sticky error (allocation failure) left by the run
     const std::string msg = p->err;
     try {
@@ -4192,10 +4218,10 @@ int ra_relation_dump_full(ra_program* p, int rel, uint64_t* host_rows, uint64_t 
         }
         const u64 *k, *v;
         u64 n;
-        version_rows(p, r, RA_FULL, &k, &v, &n);
-        u64 m = std::min<u64>(n, cap_rows);
+        u64 m = std::min<u64>(r.full_n, cap_rows);
         if (rows_out) *rows_out = m;
         if (!m || !host_rows) return;
+        version_rows(p, r, RA_FULL, &k, &v, &n, true, false);
         u64* rows;
         dev_alloc(p, &rows, m * (r.arity + 1));
         rows_unpack<<<grid_for(m), kThreads, 0, p->stream>>>(k, v, m, (int)r.arity, p->bits, rows);
@@ -4206,7 +4232,7 @@ int ra_relation_dump_full(ra_program* p, int rel, uint64_t* host_rows, uint64_t 
             ~Free() { dev_free(p, q); }
         } free_rows{p, &rows};
         rows_to_host(p, host_rows, rows, m * (r.arity + 1) * 8);
-        check_sorts(p);
+        check_sorts(p, &r);
     });
 }
 

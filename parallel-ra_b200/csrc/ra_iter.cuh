@@ -1526,7 +1526,7 @@ template <typename Timeout>
 __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ src_k, const u64* __restrict__ src_v,
                                            u64* __restrict__ dk, u64* __restrict__ dv, u64 n, int shift,
                                            const u64* __restrict__ counts, u32* __restrict__ tile_ctr,
-                                           u64* __restrict__ status, u32 tag, Timeout timeout)
+                                           u64* __restrict__ status, u32 tag, u64 limit, Timeout timeout)
 {
     const u64 ntiles = (n + kSortTile - 1) / kSortTile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1563,12 +1563,13 @@ __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ 
             long t = (long)tile - 1;
             u64 spins = 0;
             while (t >= 0) {
+                if (spins >= limit) {
+                    timeout();
+                    break;
+                }
                 const u64 sv = st_read(status + (u64)t * kRadix + d);
                 if (st_tag(sv) != (tag & 0xffffffu) || st_flag(sv) == 0) {
-                    if (++spins > kSpinLimit) {
-                        timeout();
-                        break;
-                    }
+                    spins++;
                     continue;
                 }
                 excl += st_val(sv);
@@ -1705,7 +1706,7 @@ __global__ void __launch_bounds__(kThreads) sort_pass_kernel(IterCtl* __restrict
     }
     sort_tiles(S, a.src_k, a.src_v, dk, dv, n, fits ? a.last_shift : a.shift, ctl->sort_hist[a.rel][pass],
                tile_counter(ctl, tile_slot),
-               status, iter_tag(ctl, tile_slot), [&] { atomicOr(&ctl->flags, kFlagTimeout); });
+               status, iter_tag(ctl, tile_slot), kSpinLimit, [&] { atomicOr(&ctl->flags, kFlagTimeout); });
 }
 
 // A whole array's radix sort (loading, sorted views): every pass's digit counts in one read,
@@ -1736,15 +1737,21 @@ __global__ void __launch_bounds__(kThreads) sort_counts_kernel(const u64* __rest
     }
 }
 
+// A look-back that gives up (after `limit` polls) tells the host, and the sort's later passes: a
+// pass that lacks some of its prefixes writes within the array, but leaves rows of other digits than
+// were counted, which the next pass would place beyond it.
 __global__ void __launch_bounds__(kThreads) sort_array_kernel(const u64* __restrict__ src_k, const u64* __restrict__ src_v,
                                                               u64* __restrict__ dk, u64* __restrict__ dv, u64 n,
                                                               int shift, const u64* __restrict__ counts,
                                                               u32* __restrict__ tile_ctr, u64* __restrict__ status,
-                                                              u32 tag, u64* host_timeout)
+                                                              u32 tag, u64 limit, u64* gave_up, u64* host_timeout)
 {
     __shared__ SortSmem S;
-    sort_tiles(S, src_k, src_v, dk, dv, n, shift, counts, tile_ctr, status, tag,
-               [&] { *(volatile u64*)host_timeout = 1; });
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile u64*)gave_up)) return;
+    sort_tiles(S, src_k, src_v, dk, dv, n, shift, counts, tile_ctr, status, tag, limit, [&] {
+        *(volatile u64*)gave_up = 1;
+        *(volatile u64*)host_timeout = 1;
+    });
 }
 
 __global__ void scc_start_kernel(IterCtl* __restrict__ ctl) { ctl->t_start = global_ns(); }

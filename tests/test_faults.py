@@ -142,3 +142,73 @@ def test_sliced_iteration_under_a_memory_cap():
     assert np.array_equal(got, free.dump_full(fr["T"]))   # the same log, ids included
     assert free.stats().sliced_iterations == 0
 
+
+
+def raises_timeout(call):
+    with pytest.raises(P.RAError) as e:
+        call()
+    assert e.value.status == P.engine.E_TIMEOUT
+
+
+@pytest.fixture
+def sorts_give_up(monkeypatch):
+    """A program whose array sorts give up: every look-back of a sort over more than one tile
+    (2,048 rows) ends without a poll."""
+    def make(**kw):
+        monkeypatch.setenv("RA_SORT_POLLS", "0")
+        p = P.Program(0, **kw)
+        monkeypatch.delenv("RA_SORT_POLLS")
+        return p
+    return make
+
+
+@pytest.mark.parametrize("n,dup", [(20_000, False), (20_000, True), (300_000, False)])
+def test_a_load_whose_sort_gives_up(sorts_give_up, n, dup):
+    rng = np.random.default_rng(n)
+    rows = np.zeros((n, 3), dtype=np.uint64)
+    rows[:, :2] = rng.integers(0, 50 if dup else 1 << 20, size=(n, 2))
+    rows[:, 2] = np.arange(n)
+    p = sorts_give_up()
+    rels = P.programs.build_tc(p, rows)
+    raises_timeout(lambda: p.execute(1))
+    small = tc_rows()
+    p.load_rows(rels["G"], small)                    # within a tile: nothing to look back to
+    p.execute(1)
+    o = O.OracleProgram()
+    P.programs.build_tc(o, small)
+    o.execute(1)
+    assert p.history() == o.history()
+
+
+def test_a_read_whose_sort_gives_up(sorts_give_up, tmp_path):
+    rows = tc_rows(1500, 2000, 2)
+    p = sorts_give_up()
+    rels = P.programs.build_tc(p, rows)
+    p.execute(1)
+    for _ in range(2):                               # no sorted copy is kept from the first call
+        raises_timeout(lambda: p.dump_full(rels["T"]))
+    p.set_checkpoint(str(tmp_path / "cp"), 1)
+    raises_timeout(lambda: p.execute(1))
+    dumped = [os.path.join(d, f) for d, _, fs in os.walk(tmp_path) for f in fs if f == "T_full"]
+    assert all(os.path.getsize(f) <= 2048 * 24 for f in dumped)   # dumps within a tile only
+
+
+@pytest.mark.parametrize("ids", [P.engine.IDS_EMISSION, P.engine.IDS_REFERENCE])
+def test_a_join_whose_sort_gives_up(sorts_give_up, ids):
+    """The closure's rows, derived in another order than they are joined in, feed a second SCC:
+    as the sorted inner side of a join (its index is counted from the keys), and, in the
+    reference's order, as its outer side."""
+    p = sorts_give_up(id_order=ids)
+    rels = P.programs.build_tc(p, tc_rows(1500, 2000, 2))
+    X = p.relation(1, 2, 258, "X", P.engine.FULL)
+    p.load_rows(X, np.empty((0, 3), dtype=np.uint64))
+    more = p.scc(True, 3)
+    p.add_relation(more, rels["T"], ids == P.engine.IDS_REFERENCE)
+    p.add_relation(more, X, True)
+    if ids == P.engine.IDS_REFERENCE:
+        p.join(more, X, rels["T"], P.engine.DELTA, rels["G"], P.engine.FULL, [3, 1])
+    else:
+        p.join(more, X, rels["G"], P.engine.FULL, rels["T"], P.engine.FULL, [3, 1])
+    p.depend(0, more)                                # the closure's SCC
+    raises_timeout(lambda: p.execute(1))
+    raises_timeout(lambda: p.execute(1))             # the failed run left the program as it was
