@@ -30,12 +30,11 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
-#include <condition_variable>
 #include <functional>
-#include <mutex>
 #include <thread>
 #include <fstream>
 #include <string>
+#include <sys/mman.h>
 #include <sys/stat.h>
 #include <unistd.h>
 #include <unordered_map>
@@ -354,131 +353,65 @@ u64 read_scalar(ra_program* p, const u64* dptr)
     return p->hscalar[0];
 }
 
-// Pinned staging of large reads to the host, shared by the process's programs: 12 MB, made
-// by the first such read (pinning costs milliseconds), freed with the last program.  One
-// read uses it at a time; another one meanwhile takes the plain copy.
-constexpr u64 kRingChunk = 2u << 20;
-constexpr int kRingChunks = 6;
-constexpr int kRingThreads = 4;
-constexpr u64 kRingBytes = 12u << 20;   // reads below are plain copies
-
-struct HostRing {
-    std::mutex busy;          // held while a read uses (or frees) the buffer
-    std::mutex count_mu;
-    int programs = 0;
-    char* buf = nullptr;
-    void add()
-    {
-        std::lock_guard<std::mutex> lk(count_mu);
-        programs++;
+// Are pages of the caller's memory still to be made?  (Looks at 16 of them.  No for page-locked,
+// managed and device memory.)
+bool fresh_pages(const void* dst, u64 bytes)
+{
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    void remove()
-    {
-        std::lock_guard<std::mutex> lk(count_mu);
-        if (--programs) return;
-        std::lock_guard<std::mutex> use(busy);
-        if (buf) cudaFreeHost(buf);
-        buf = nullptr;
+    if (at.type != cudaMemoryTypeUnregistered) return false;
+    const u64 page = (u64)sysconf(_SC_PAGESIZE);
+    for (u64 i = 0; i < 16; i++) {
+        unsigned char here = 1;
+        const u64 addr = ((u64)dst + bytes / 16 * i) & ~(page - 1);
+        if (mincore((void*)addr, page, &here) != 0) return false;
+        if (!(here & 1)) return true;
     }
-};
-HostRing g_ring;
+    return false;
+}
 
-// Device bytes to pageable host memory, complete on return.  A plain copy is bound by one
-// thread of the driver that moves staged bytes into the caller's pages, faults of fresh
-// pages included.  Large reads land chunk by chunk in a pinned ring, and four threads move
-// the chunks on.  Measured (16-core host): 45 MB of fresh rows 10.7 -> 3.4 ms, of touched
-// ones 2.8 -> 2.0; 100 MB fresh 22.5 -> 7.6; 16 MB 1.45 -> 1.0; 8 MB 0.72 -> 0.92, so these stay
-// plain.  Chunks of 512 KB and eight threads: 30 MB touched 6.3 ms against 1.4 (the threads
-// meet in one huge page, and at the lock).
+// Device bytes to host memory, complete on return.  A plain copy into fresh pageable memory is
+// bound by the driver's one thread, which takes a page fault for each page it fills; for large
+// reads four threads have the kernel make the pages, in order, 2 MB at a time, while the copy goes on.
+// Measured (16-core host), plain -> so: 45 MB of fresh 4 KB pages 20.5 -> 4.6 ms, of fresh 2 MB ones
+// 9.1 -> 3.5; 12 MB 5.5 -> 2.1 and 2.4 -> 1.9; 8 MB of 2 MB pages 1.7 -> 1.9, so these stay plain.  Six
+// threads meet at the address space's lock (45 MB: 10.9 and 8.1 ms).  Pages that are there already
+// would gain nothing (45 MB: 2.3 ms either way).
+constexpr u64 kPopulateBytes = 12u << 20;
+constexpr u64 kPopulateBlock = 2u << 20;
+constexpr int kPopulateThreads = 4;
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
 void rows_to_host(ra_program* p, void* dst, const void* src, u64 bytes)
 {
-    std::unique_lock<std::mutex> use(g_ring.busy, std::defer_lock);
-    bool ring = bytes >= kRingBytes && std::thread::hardware_concurrency() >= 2 * kRingThreads && use.try_lock();
-    if (ring && !g_ring.buf && cudaHostAlloc((void**)&g_ring.buf, kRingChunk * kRingChunks, cudaHostAllocPortable) !=
-                                   cudaSuccess) {
-        cudaGetLastError();
-        g_ring.buf = nullptr;
-        ring = false;
-    }
-    struct Events {
-        cudaEvent_t e[kRingChunks] = {};
-        ~Events()
-        {
-            for (cudaEvent_t v : e)
-                if (v) cudaEventDestroy(v);
-        }
-    } ev;
-    for (int i = 0; i < kRingChunks && ring; i++) CK(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming));
-    if (!ring) {
-        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, p->stream));
-        CK(cudaStreamSynchronize(p->stream));
-        return;
-    }
-    char* const buf = g_ring.buf;
-    const u64 chunks = (bytes + kRingChunk - 1) / kRingChunk;
-    auto move_on = [&](u64 i) {
-        const u64 at = i * kRingChunk;
-        std::memcpy((char*)dst + at, buf + (i % kRingChunks) * kRingChunk, std::min(kRingChunk, bytes - at));
-    };
-    std::vector<char> moved(chunks, 0);
-    std::mutex mu;
-    std::condition_variable more, room;   // a chunk landed (or the read ended); a chunk was moved on
-    u64 ready = 0, taken = 0;             // chunks landed, chunks a thread has taken
-    bool end = false;
-    auto work = [&]() {
-        std::unique_lock<std::mutex> lk(mu);
-        for (;;) {
-            more.wait(lk, [&] { return end || taken < ready; });
-            if (taken >= ready) return;
-            const u64 i = taken++;
-            lk.unlock();
-            move_on(i);
-            lk.lock();
-            moved[i] = 1;
-            room.notify_one();
-        }
-    };
     std::vector<std::thread> pool;
-    try {
-        pool.reserve(kRingThreads);
-        for (int t = 0; t < kRingThreads; t++) pool.emplace_back(work);
-    } catch (...) {   // as many threads as could be had; none: this one moves the chunks
-    }
-    cudaError_t err = cudaSuccess;
-    u64 issued = 0;
-    for (u64 landed = 0; landed < chunks && err == cudaSuccess; landed++) {
-        while (issued < chunks && issued < landed + kRingChunks && err == cudaSuccess) {
-            if (issued >= (u64)kRingChunks && !pool.empty()) {   // its slot's last chunk must have left
-                std::unique_lock<std::mutex> lk(mu);
-                const u64 old = issued - kRingChunks;
-                if (issued > landed && !moved[old]) break;   // other chunks are in flight: see to those
-                room.wait(lk, [&] { return moved[old] != 0; });
-            }
-            const u64 at = issued * kRingChunk, slot = issued % kRingChunks;
-            err = cudaMemcpyAsync(buf + slot * kRingChunk, (const char*)src + at, std::min(kRingChunk, bytes - at),
-                                  cudaMemcpyDeviceToHost, p->stream);
-            if (err == cudaSuccess) err = cudaEventRecord(ev.e[slot], p->stream);
-            issued++;
+    std::atomic<u64> next{0};
+    if (bytes >= kPopulateBytes && std::thread::hardware_concurrency() >= 2 * kPopulateThreads &&
+        fresh_pages(dst, bytes)) {
+        const u64 page = (u64)sysconf(_SC_PAGESIZE);
+        const u64 first = ((u64)dst + page - 1) & ~(page - 1), last = ((u64)dst + bytes) & ~(page - 1);
+        try {
+            pool.reserve(kPopulateThreads);
+            for (int t = 0; t < kPopulateThreads; t++)
+                pool.emplace_back([&next, first, last] {
+                    for (;;) {
+                        const u64 at = first + next.fetch_add(kPopulateBlock);
+                        // a kernel without the call leaves the faults to the copy
+                        if (at >= last || madvise((void*)at, std::min(kPopulateBlock, last - at), MADV_POPULATE_WRITE))
+                            return;
+                    }
+                });
+        } catch (...) {   // as many threads as could be had
         }
-        if (err == cudaSuccess) err = cudaEventSynchronize(ev.e[landed % kRingChunks]);
-        if (err != cudaSuccess) break;
-        if (pool.empty()) {
-            move_on(landed);
-            continue;
-        }
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            ready = landed + 1;
-        }
-        more.notify_one();
     }
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        end = true;
-    }
-    more.notify_all();
+    cudaError_t err = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, p->stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(p->stream);
     for (std::thread& t : pool) t.join();
-    if (err != cudaSuccess) cudaStreamSynchronize(p->stream);   // no copy still writes the ring
     ck(p, err, "rows to host");
 }
 
@@ -3630,7 +3563,6 @@ int ra_program_create(int device, ra_program** out)
         delete p;
         return st;
     }
-    g_ring.add();
     *out = p;
     return RA_OK;
 }
@@ -3700,7 +3632,6 @@ int ra_program_destroy(ra_program* p)
     }
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
-    g_ring.remove();
     return RA_OK;
 }
 

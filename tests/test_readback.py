@@ -1,9 +1,13 @@
-"""Rows read back to host memory: small ones by one copy, larger ones (12 MB up) chunk by chunk
-through a pinned ring and several threads; every size gives the loaded rows in trie order."""
+"""Rows read back to host memory: by one copy, into large fresh memory (12 MB up) while several
+threads make its pages; every size gives the loaded rows in trie order."""
+import ctypes as C
+import mmap
 import threading
+import time
 
 import numpy as np
 import pytest
+import torch
 
 import parallel_ra_b200 as P
 
@@ -37,7 +41,7 @@ def test_sizes_around_the_ring(width, top):
 
 
 def test_two_programs_read_at_once():
-    # one read has the ring, the other one goes without
+    # both while threads make their pages
     out, progs = {}, []
     for k in range(2):
         p = P.Program(0)
@@ -60,3 +64,76 @@ def test_two_programs_read_at_once():
         want = rows[np.argsort(rows[:, 0])]
         assert all(np.array_equal(g, want) for g in out[k])
         p.close()
+
+
+def loaded(nbytes):
+    p = P.Program(0)
+    r = p.relation(1, 2, 7, "R")
+    rows = rows_of(nbytes, 3, 1000, 5)
+    p.load_rows(r, rows)
+    p.execute(1)
+    return p, r, rows[np.argsort(rows[:, 0])]
+
+
+def read_into(p, r, address, n):
+    got = C.c_uint64()
+    t = time.perf_counter()
+    assert p._L.ra_relation_dump_full(p.handle, r, C.cast(address, C.POINTER(C.c_uint64)), n, C.byref(got)) == 0
+    assert got.value == n
+    return time.perf_counter() - t
+
+
+def mapped(nbytes, how):
+    """Fresh memory of nbytes, its address off the start of a page (and an object that keeps it)."""
+    m = mmap.mmap(-1, nbytes + 8192)
+    if how == "some touched":
+        m[:nbytes // 3] = b"\1" * (nbytes // 3)
+    if how == "all touched":
+        m[:] = b"\1" * len(m)
+    return C.addressof(C.c_char.from_buffer(m)) + 40, m
+
+
+@pytest.mark.parametrize("how", ["fresh", "some touched", "all touched", "page-locked"])
+@pytest.mark.parametrize("nbytes", [6 * CHUNK, 11 * CHUNK + 24, 40 << 20])
+def test_memory_of_every_kind(how, nbytes):
+    p, r, want = loaded(nbytes)
+    if how == "page-locked":
+        keep = torch.zeros(want.size, dtype=torch.int64, pin_memory=True)
+        at = keep.data_ptr()
+    else:
+        at, keep = mapped(want.nbytes, how)
+    for _ in range(2):
+        read_into(p, r, at, len(want))
+        got = np.ctypeslib.as_array(C.cast(at, C.POINTER(C.c_uint64)), want.shape)
+        assert np.array_equal(got, want)
+    p.close()
+
+
+def test_page_locked_rows_are_read_by_one_copy():
+    """45 MB into page-locked rows take the time of the copy (half as much again for the rest of the call)."""
+    p, r, want = loaded(45 << 20)
+    host = torch.empty(want.size, dtype=torch.int64, pin_memory=True)
+    dev = torch.zeros(want.size, dtype=torch.int64, device="cuda")
+    copies = []
+    for _ in range(10):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        host.copy_(dev)
+        torch.cuda.synchronize()
+        copies.append(time.perf_counter() - t)
+    reads = [read_into(p, r, host.data_ptr(), len(want)) for _ in range(10)]
+    assert min(reads) < 1.5 * min(copies)
+    p.close()
+
+
+def test_a_program_s_first_read_costs_no_set_up():
+    """Programs that are made for one read: the first read takes about as long as the next (the
+    first of a process aside), whatever was read or closed before."""
+    first, again = [], []
+    at, keep = mapped(15 << 20, "all touched")
+    for _ in range(4):
+        p, r, want = loaded(14 << 20)
+        first.append(read_into(p, r, at, len(want)))
+        again += [read_into(p, r, at, len(want)) for _ in range(3)]
+        p.close()
+    assert min(first) < 2 * min(again) + 1e-3
