@@ -87,9 +87,11 @@ __global__ void __launch_bounds__(1024) rows_max_small_kernel(const u64* __restr
 // The whole load of a small relation by one block: rows packed, sorted by (key, id) in shared
 // memory (bitonic; 16 bytes per row), exact repetitions dropped, the result written to the log
 // and to the copy that a reset restores; row count and whether two rows share data columns go
-// straight to page-locked host memory.  A radix sort takes five launches per 8 key bits and two
-// round trips here; bound by the network's stages.  390 rows: 12 us.
-constexpr u32 kLoadSmall = 8192;
+// straight to page-locked host memory.  A radix sort takes a launch per 8 key bits and two round
+// trips; bound by the network's stages.  390 rows: 12 us.  Load and run of distinct rows of 40 bits,
+// so against by radix sort: 512 rows 60 and 120 us, 2,048 104 and 137, 4,096 (the line; twice
+// the rows are two stages and a longer stage) 132 and 155, 4,097 204 and 146, 8,192 233 and 155.
+constexpr u32 kLoadSmall = 4096;
 __global__ void __launch_bounds__(1024) load_small_kernel(const u64* __restrict__ rows, u32 n, int arity, int bits,
                                                           u64* __restrict__ keys, u64* __restrict__ ids,
                                                           u64* __restrict__ lkeys, u64* __restrict__ lids,

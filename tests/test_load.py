@@ -1,5 +1,7 @@
 """Loading: small relations (one block sorts them and drops repetitions) and larger ones, at the
 edges between the two, and small and larger join indexes, against numpy and the oracle."""
+import time
+
 import numpy as np
 import pytest
 
@@ -26,6 +28,30 @@ def test_loaded_rows_are_sorted_and_distinct(n, kind):
         assert np.array_equal(p.dump_full(r), np.unique(rows, axis=0))
         p.execute(1)
         assert np.array_equal(p.dump_full(r), np.unique(rows, axis=0))
+
+
+@pytest.mark.parametrize("n", [4095, 4096])
+@pytest.mark.parametrize("kind", ["distinct", "shared_data", "repeated"])
+def test_rows_at_the_line_between_the_loads(n, kind):
+    test_loaded_rows_are_sorted_and_distinct(n, kind)
+
+
+def test_a_row_more_is_not_the_faster_load():
+    """The one-block load ends where the sort over the grid takes over with a gain."""
+    best = {}
+    for n in (4096, 4097, 8192, 8193):
+        rows = np.random.default_rng(n).integers(0, 1 << 20, size=(n, 3), dtype=np.uint64)
+        p = P.Program(0)
+        r = p.relation(1, 2, 9, "R")
+        times = []
+        for _ in range(40):
+            t = time.perf_counter()
+            p.load_rows(r, rows)
+            p.execute(1)
+            times.append(time.perf_counter() - t)
+        best[n] = min(times)
+        p.close()
+    assert best[4096] < 1.2 * best[4097] and best[8192] < 1.2 * best[8193], best
 
 
 # join indexes: rows up to / above 4,096, key ranges up to / above 2^16, a row of more than 4,096
