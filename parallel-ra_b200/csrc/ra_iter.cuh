@@ -635,7 +635,10 @@ __device__ __forceinline__ void join_tiles(JoinSmem& S, IterCtl* __restrict__ ct
                     mine[k] = tag_base + at[k];
                     if (valid[k] && !(kSplit && bs.seen)) cand[cbase + at[k]] = key[k];
                 }
-                if (kSplit && bs.seen) {
+                // never taken without kSplit, but compiled: where this branch was left out, the claims of
+                // repeated candidates took longer (a closure of 145 grids of 30 x 30 values, half of
+                // its candidates repeated: 5.37 ms of iterations against 4.80)
+                if (bs.seen) {
 #pragma unroll
                     for (int k = 0; k < kClaimBatch; k++)
                         if (valid[k]) bit_claim(bs, key[k], bits, ctl);
