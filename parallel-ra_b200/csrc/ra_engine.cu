@@ -2374,11 +2374,22 @@ void run_scc_device(ra_program* p, Scc& s, DevScc& d)
     p->history.insert(p->history.end(), hist.begin(), hist.end());
 }
 
+// One allocation, cut into arrays: room for count Ts, and with `all` set, their address.
+struct BufferCut {
+    u8* all = nullptr;
+    u64 used = 0;
+    template <typename T>
+    void operator()(T** at, u64 count)
+    {
+        if (all) *at = (T*)(all + used);
+        used += (count * sizeof(T) + 255) & ~255ull;
+    }
+};
+
 // Device buffers of one dense evaluation, freed on every exit.
 struct DenseBufs {
     ra_program* p;
-    u8* all = nullptr;      // one allocation, cut into the arrays below
-    u64 used = 0;
+    BufferCut cut;
     u32* known = nullptr;
     u32* delta0 = nullptr;
     u64* row_new = nullptr;
@@ -2392,15 +2403,8 @@ struct DenseBufs {
     explicit DenseBufs(ra_program* pp) : p(pp) {}
     ~DenseBufs()
     {
-        dev_free(p, &all);
+        dev_free(p, &cut.all);
         dev_free(p, &meta);
-    }
-    // room for count Ts in the allocation: with `all` set, their address
-    template <typename T>
-    void cut(T** at, u64 count)
-    {
-        if (all) *at = (T*)(all + used);
-        used += (count * sizeof(T) + 255) & ~255ull;
     }
 };
 constexpr u64 kDenseTotal = 1, kDenseCounters = 2, kDenseLevels0 = 10;   // words of DenseBufs::meta; flags in word 0
@@ -2553,8 +2557,8 @@ bool run_scc_dense(ra_program* p, Scc& s)
     DenseBufs B(p);
     for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
         if (pass) {
-            dev_alloc(p, &B.all, B.used);
-            B.used = 0;
+            dev_alloc(p, &B.cut.all, B.cut.used);
+            B.cut.used = 0;
         }
         B.cut(&B.known, words);
         if (!all_delta) B.cut(&B.delta0, words);
@@ -2733,18 +2737,15 @@ bool closure_shape(ra_program* p, const Scc& s, JoinPlan& jp)
 // Device buffers of one sparse row closure, freed on every exit.
 struct SparseBufs {
     ra_program* p;
-    u64 *first = nullptr, *adj = nullptr, *tile_at = nullptr, *tile_lv = nullptr, *ctr = nullptr, *base = nullptr;
-    u32 *target = nullptr, *queue = nullptr, *arena = nullptr, *levels = nullptr, *pos = nullptr, *tile_nlv = nullptr;
-    u32 *block_lv = nullptr, *flags = nullptr, *big_queue = nullptr;
-    u16 *warp_lv = nullptr, *big_table = nullptr;
+    // the large ones apart, so that the pool finds them room among blocks given back to it
+    BufferCut fixed, levels;
+    u32 *queue = nullptr, *table = nullptr, *arena = nullptr;
     explicit SparseBufs(ra_program* pp) : p(pp) {}
     ~SparseBufs()
     {
-        for (u64** q : {&first, &adj, &tile_at, &tile_lv, &ctr, &base}) dev_free(p, q);
-        for (u32** q : {&target, &queue, &arena, &levels, &pos, &tile_nlv, &block_lv, &flags, &big_queue})
-            dev_free(p, q);
-        dev_free(p, &warp_lv);
-        dev_free(p, &big_table);
+        dev_free(p, &fixed.all);
+        dev_free(p, &levels.all);
+        for (u32** b : {&queue, &table, &arena}) dev_free(p, b);
     }
 };
 
@@ -2769,6 +2770,7 @@ bool run_scc_sparse(ra_program* p, Scc& s)
     version_rows(p, S, RA_FULL, &sk, &sv, &sn);
     if (sn == 0 || n > 16 * sn + (1u << 18)) return false;   // per-value arrays would dwarf the input
     const u64* scsr = version_csr(p, S, RA_FULL);
+    if (S.csr_full_longest > kSpBigQueue) return false;   // a tile that reaches that value is too large
     const u64 n_stored = R.delta_n;
     SparseBufs B(p);
     SparseArgs a{};
@@ -2780,75 +2782,81 @@ bool run_scc_sparse(ra_program* p, Scc& s)
     a.n_delta = n_stored;
     a.arena_cap = std::max<u64>(p->sp_arena_hint, 24 * sn + (1u << 20));
     a.levels_cap = std::max<u64>(p->sp_levels_hint, 48ull * a.tiles + (1u << 16));
-    static int occ = 0;
-    if (!occ) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sparse_search_kernel, kSpWarps * 32, 0));
+    int occ = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sparse_search_kernel, kSpWarps * 32, 0));
+    CK(cudaFuncSetAttribute(sparse_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpBigSmem));
     const int grid = (int)std::min<u64>((u64)kSms * std::max(occ, 1), (a.tiles + kSpWarps - 1) / kSpWarps);
-    a.big = std::min<u32>(kSpBig, 16 + a.tiles / 64);
-    std::vector<u64> total(kSpLevels), hc(4);
-    u32 fl = 0;
+    const u64 warps = (u64)grid * kSpWarps;
+    a.large = std::max<u32>(4 * kSpBig, a.tiles / 32);
+    // flags, counters and level totals, read back together
+    constexpr u64 kMetaCtr = 16, kMetaLevels = kMetaCtr + kSpCtrWords, kMetaWords = kMetaLevels + kSpLevels;
+    u64 *meta = nullptr, *base_dev = nullptr;
+    u32* pos = nullptr;
+    const u64 *total = nullptr, *hc = nullptr;
     try {
-        dev_alloc(p, &B.first, a.tiles + 1);
-        dev_alloc(p, &B.adj, n);
-        dev_alloc(p, &B.target, sn);
-        dev_alloc(p, &B.queue, (u64)grid * kSpWarps * kSpQueue);
-        dev_alloc(p, &B.warp_lv, (u64)grid * kSpWarps * kSpLevels);
-        dev_alloc(p, &B.big_queue, (u64)a.big * kSpBigQueue);
-        dev_alloc(p, &B.big_table, (u64)a.big * kSpBigSlots);
-        dev_alloc(p, &B.tile_at, a.tiles);
-        dev_alloc(p, &B.tile_lv, a.tiles);
-        dev_alloc(p, &B.tile_nlv, a.tiles);
-        dev_alloc(p, &B.block_lv, (u64)a.blocks * kSpLevels);
-        dev_alloc(p, &B.ctr, 5 + kSpLevels);
-        dev_alloc(p, &B.base, kSpLevels);
-        dev_alloc(p, &B.flags, 1);
-        a.first = B.first;
-        a.adj = B.adj;
-        a.target = B.target;
+        for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
+            if (pass) {
+                dev_alloc(p, &B.fixed.all, B.fixed.used);
+                B.fixed.used = 0;
+            }
+            B.fixed(&a.first, a.tiles + 1);
+            B.fixed(&a.adj, n);
+            B.fixed(&a.target, sn);
+            B.fixed(&a.warp_lv, warps * kSpLevels);
+            B.fixed(&a.big_tile, kSpBigMost);
+            B.fixed(&a.tile_at, a.tiles);
+            B.fixed(&a.tile_lv, a.tiles);
+            B.fixed(&a.tile_nlv, a.tiles);
+            B.fixed(&a.block_lv, (u64)a.blocks * kSpLevels);
+            B.fixed(&meta, kMetaWords);
+            B.fixed(&base_dev, kSpLevels);
+        }
+        dev_alloc(p, &B.queue, warps * kSpQueue);
+        dev_alloc(p, &B.table, warps * 4 * kSpBuckets);
         a.queue = B.queue;
-        a.warp_lv = B.warp_lv;
-        a.big_queue = B.big_queue;
-        a.big_table = B.big_table;
-        a.tile_at = B.tile_at;
-        a.tile_lv = B.tile_lv;
-        a.tile_nlv = B.tile_nlv;
-        a.block_lv = B.block_lv;
-        a.ctr = B.ctr;
-        a.level_total = B.ctr + 5;
-        a.flags = B.flags;
-        CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
+        a.table = B.table;
+        a.flags = (u32*)meta;
+        a.ctr = meta + kMetaCtr;
+        a.level_total = meta + kMetaLevels;
+        CK(cudaMemsetAsync(meta, 0, kMetaWords * 8, p->stream));
         sparse_adj_kernel<<<grid_for(std::max(n, sn)), kThreads, 0, p->stream>>>(a, scsr, sk, sn);
         LAUNCHED();
         sparse_bounds_kernel<<<grid_for(n_stored + 1), kThreads, 0, p->stream>>>(a);
         LAUNCHED();
         for (int round = 0;; round++) {
             dev_free(p, &B.arena);
-            dev_free(p, &B.levels);
-            dev_free(p, &B.pos);
+            dev_free(p, &B.levels.all);
             dev_alloc(p, &B.arena, a.arena_cap);
-            dev_alloc(p, &B.levels, a.levels_cap);
-            dev_alloc(p, &B.pos, a.levels_cap);
             a.arena = B.arena;
-            a.levels = B.levels;
-            CK(cudaMemsetAsync(B.block_lv, 0, (u64)a.blocks * kSpLevels * 4, p->stream));
-            CK(cudaMemsetAsync(B.ctr, 0, (5 + kSpLevels) * 8, p->stream));
+            for (int pass = 0; pass < 2; pass++) {
+                if (pass) dev_alloc(p, &B.levels.all, B.levels.used);
+                B.levels.used = 0;
+                B.levels(&a.levels, a.levels_cap);
+                B.levels(&pos, a.levels_cap);
+            }
+            CK(cudaMemsetAsync(a.block_lv, 0, (u64)a.blocks * kSpLevels * 4, p->stream));
             sparse_search_kernel<<<grid, kSpWarps * 32, 0, p->stream>>>(a);
+            LAUNCHED();
+            sparse_big_kernel<<<kSms, kSpBigThreads, kSpBigSmem, p->stream>>>(a);
             LAUNCHED();
             sparse_scan_kernel<<<kSpLevels / kWarps, kThreads, 0, p->stream>>>(a);
             LAUNCHED();
-            CK(cudaMemcpyAsync(&fl, B.flags, 4, cudaMemcpyDeviceToHost, p->stream));
-            CK(cudaMemcpyAsync(hc.data(), B.ctr, 4 * 8, cudaMemcpyDeviceToHost, p->stream));
-            CK(cudaMemcpyAsync(total.data(), a.level_total, kSpLevels * 8, cudaMemcpyDeviceToHost, p->stream));
+            u64* got = host_words(p, kMetaWords);
+            CK(cudaMemcpyAsync(got, meta, kMetaWords * 8, cudaMemcpyDeviceToHost, p->stream));
             CK(cudaStreamSynchronize(p->stream));
-            if ((fl & ~kSpArena) || hc[1] >> 32) return false;   // positions within a level are 32 bits
+            const u32 fl = (u32)got[0];
+            hc = got + kMetaCtr;
+            total = got + kMetaLevels;
+            if ((fl & ~kSpArena) || hc[kSpArenaN] >> 32) return false;   // positions within a level are 32 bits
             if (!(fl & kSpArena)) break;
             if (round) return false;
-            a.arena_cap = std::max(a.arena_cap, hc[1]);   // the whole search's needs are known
-            a.levels_cap = std::max(a.levels_cap, hc[2]);
-            CK(cudaMemsetAsync(B.flags, 0, 4, p->stream));
+            a.arena_cap = std::max<u64>(a.arena_cap, hc[kSpArenaN]);   // the whole search's needs are known
+            a.levels_cap = std::max<u64>(a.levels_cap, hc[kSpLevelN]);
+            CK(cudaMemsetAsync(meta, 0, kMetaWords * 8, p->stream));
         }
-        p->sp_arena_hint = hc[1] + hc[1] / 8;
-        p->sp_levels_hint = hc[2] + hc[2] / 8;
-        ensure_log(p, R, n_stored + hc[1]);
+        p->sp_arena_hint = hc[kSpArenaN] + hc[kSpArenaN] / 8;
+        p->sp_levels_hint = hc[kSpLevelN] + hc[kSpLevelN] / 8;
+        ensure_log(p, R, n_stored + hc[kSpArenaN]);
     } catch (const ra_error& e) {
         if (e.status != RA_E_OOM) throw;
         p->err.clear();   // no room for the scratch
@@ -2856,23 +2864,24 @@ bool run_scc_sparse(ra_program* p, Scc& s)
         return false;
     }
     u64 L = 0, sum = 0;
-    std::vector<u64> base(kSpLevels, 0);
+    std::vector<u64> lv(kSpLevels, 0), base(kSpLevels, 0);
     for (; L < kSpLevels && total[L]; L++) {
+        lv[L] = total[L];
         base[L] = sum;
         sum += total[L];
     }
     if (sum) {
         const u64 id0 = ((u64)R.tag << 46) | intern_counter(p, R.tag);
-        CK(cudaMemcpyAsync(B.base, base.data(), L * 8, cudaMemcpyHostToDevice, p->stream));
-        sparse_offsets_kernel<<<a.blocks, kThreads, 0, p->stream>>>(a, B.pos);
+        CK(cudaMemcpyAsync(base_dev, base.data(), L * 8, cudaMemcpyHostToDevice, p->stream));
+        sparse_offsets_kernel<<<a.blocks, kThreads, 0, p->stream>>>(a, pos);
         LAUNCHED();
         sparse_place_kernel<<<(int)std::min<u64>((a.tiles + kWarps - 1) / kWarps, kSms * 8), kThreads, 0, p->stream>>>(
-            a, B.pos, B.base, R.keys + n_stored, R.ids + n_stored, sum, id0);
+            a, pos, base_dev, R.keys + n_stored, R.ids + n_stored, sum, id0);
         LAUNCHED();
         CK(cudaStreamSynchronize(p->stream));   // the scratch goes when this returns
     }
-    p->stats.join_candidates += hc[3];
-    finish_closure_scc(p, s, s.rules[0].out, R, n_stored, sum, total, L, L + 1);
+    p->stats.join_candidates += hc[kSpTried];
+    finish_closure_scc(p, s, s.rules[0].out, R, n_stored, sum, lv, L, L + 1);
     return true;
 }
 

@@ -1566,13 +1566,12 @@ __device__ __forceinline__ void sort_tiles(SortSmem& S, const u64* __restrict__ 
             long t = (long)tile - 1;
             u64 spins = 0;
             while (t >= 0) {
-                if (spins >= limit) {
-                    timeout();
-                    break;
-                }
                 const u64 sv = st_read(status + (u64)t * kRadix + d);
-                if (st_tag(sv) != (tag & 0xffffffu) || st_flag(sv) == 0) {
-                    spins++;
+                if (st_tag(sv) != (tag & 0xffffffu) || st_flag(sv) == 0 || limit == 0) {
+                    if (++spins > limit) {
+                        timeout();
+                        break;
+                    }
                     continue;
                 }
                 excl += st_val(sv);

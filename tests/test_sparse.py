@@ -1,6 +1,8 @@
 """The sparse row closure (a transitive-closure-shaped SCC over more than 65,536 values whose
 rows stay small, one warp per 16 rows) leaves what the iteration loop leaves: history,
 rows and ids; what it cannot hold goes to the loop."""
+import time
+
 import numpy as np
 import pytest
 
@@ -122,3 +124,105 @@ def test_runs_repeat_and_other_inputs_follow():
         q, rq = run(rows, loop=True)
         assert p.history() == q.history()
         assert np.array_equal(p.dump_full(rels["T"])[:, :2], q.dump_full(rq["T"])[:, :2])
+
+
+def clique(n, base=5):
+    v = np.arange(base, base + n, dtype=np.uint64)
+    e = np.stack(np.meshgrid(v, v, indexing="ij"), axis=-1).reshape(-1, 2)
+    return e[e[:, 0] != e[:, 1]]
+
+
+def layers(*widths):
+    """Every node of a layer to every node of the next; the first layer is a tile's rows."""
+    first = np.cumsum((16,) + widths)
+    out = []
+    for k in range(len(widths) - 1):
+        a, b = (np.arange(first[i], first[i + 1], dtype=np.uint64) for i in (k, k + 1))
+        out.append(np.stack(np.meshgrid(a, b, indexing="ij"), axis=-1).reshape(-1, 2))
+    return np.concatenate(out)
+
+
+def grid(k):
+    v = np.arange(16, 16 + k * k, dtype=np.uint64).reshape(k, k)
+    return np.concatenate([np.stack([v[:-1].ravel(), v[1:].ravel()], 1), np.stack([v[:, :-1].ravel(), v[:, 1:].ravel()], 1)])
+
+
+def star(leaves, more=()):
+    return np.concatenate([np.stack([np.full(leaves, 7), np.arange(1000, 1000 + leaves)], axis=1),
+                           np.array(more, dtype=np.int64).reshape(-1, 2)]).astype(np.uint64)
+
+
+def twice(edges):
+    return np.concatenate([edges, edges])
+
+
+# tuples found again and again: by the filter, the queue, a warp's table, a CTA's table
+AGAIN = {
+    "cliques_of_3": np.concatenate([clique(3, 5 * k) for k in range(3000)]),
+    "cliques_of_20": np.concatenate([clique(20, 32 * k + 3) for k in range(200)]),
+    "clique_of_32": clique(32, 16), "clique_of_33": clique(33, 16),      # 15,872 and 16,896 candidates of a tile
+    "clique_of_128": clique(128, 16), "clique_of_129": clique(129, 16),  # 260,096 and 264,192
+    "layers_to_few": layers(16, 40, 100),
+    "layers_to_many": layers(16, 40, 300),
+    "layers_to_1024": layers(16, 1, 1024, 3, 500),
+    "grid": grid(24),
+    "larger_grid": grid(36),
+    "edges_twice": twice(er(3000, 4000, 3)) + np.uint64(1000),
+    "star_4095": star(4095), "star_4096": star(4096), "star_4097": star(4097),
+    "star_in_a_chain": star(4097, [(3, 7), (2, 3), (7, 2), (5000, 9), (5001, 9), (9, 7)]),
+    "star_edges_twice": twice(star(4000, [(1000, 3), (1001, 3), (3, 1002), (3, 4)])),
+    "hub_of_2000_leaves": layers(16, 1, 2000),
+    "32768_tuples": layers(16, 1, 2047),       # 16 rows, a hub and its leaves
+    "32784_tuples": layers(16, 1, 2048),
+    "wide_and_deep": np.concatenate([star(5000), np.array([[1000, 20_000]], dtype=np.uint64), path(900, 20_000)]),
+}
+
+
+DECLINED = ("32784_tuples",     # a tuple too many
+            "clique_of_129")    # too many candidates
+
+
+@pytest.mark.parametrize("case", sorted(AGAIN))
+def test_tuples_found_again_leave_what_the_loop_leaves(case):
+    rows = P.datagen.with_row_ids(with_top(AGAIN[case]))
+    a, ra = run(rows)
+    b, rb = run(rows, loop=True)
+    if case != "edges_twice":   # a giant component, given up or not by a rule of thumb
+        assert (a.stats().dedup_launches == 1) == (case not in DECLINED)
+    assert a.history() == b.history()
+    assert a.stats().join_candidates == b.stats().join_candidates
+    for name in ra:
+        assert np.array_equal(a.dump_full(ra[name]), b.dump_full(rb[name])), name   # ids included
+
+
+# (edges, does the sparse closure take them)
+LOST = {
+    "a_tree": (lambda: P.datagen.random_tree(200_000, 3), False),
+    "just_above_critical": (lambda: er(70_000, 73_500, 5), False),
+    "hub_of_60000": (lambda: with_top(layers(1000, 1, 60_000)), False),
+    "star_of_30000": (lambda: with_top(star(30_000)), True),
+    "cliques_of_16": (lambda: np.concatenate([clique(16, 16 * k) for k in range(4400)]), True),
+    "cliques_of_64": (lambda: np.concatenate([clique(64, 64 * k) for k in range(1100)]), False),
+    "sources_hubs_targets": (lambda: with_top(layers(300, 100, 300)), False),
+}
+
+
+@pytest.mark.parametrize("case", sorted(LOST))
+def test_no_time_is_lost_to_the_loop(case):
+    """Closures that the search gives up, or that find every tuple many times, take hardly longer
+    than by the loop alone."""
+    make, taken = LOST[case]
+    rows = P.datagen.with_row_ids(make())
+    best = []
+    for loop in (False, True):
+        p, _ = run(rows, loop)
+        if not loop:
+            assert (p.stats().dedup_launches == 1) == taken
+        times = []
+        for _ in range(5):
+            t = time.perf_counter()
+            p.execute(1)
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+        p.close()
+    assert best[0] < 1.25 * best[1] + 0.3e-3, best
