@@ -55,7 +55,7 @@ struct DenseArgs {
     u64* level_total;            // per iteration: new tuples
     u64* inst_level;             // [iteration][instance] new tuples, or null
     u64 level_cap;
-    u64* counters;               // [0], [2..4] chunks taken (per kernel shape), [1] join candidates (S rows visited),
+    u64* counters;               // [0], [2..4], [7] chunks taken (per kernel shape), [1] join candidates (S rows visited),
                                  // [5] 1 + the first key found outside its instance, [6] its relation (1: R, 2: S)
     u32* flags;
 };
@@ -300,7 +300,7 @@ constexpr int kMsRows = 32;           // rows searched together: one bit each of
 constexpr u64 kMsMaxN = 18944;        // values per instance: three words of each fit an SM's shared memory
 constexpr u32 kMsSmemQueueN = 13824;  // ... with both queues beside them; above, kMsNear entries of each are
 constexpr u32 kMsNear = 1024;
-constexpr int kMsWords = 4;           // words of a row a lane loads at a time
+constexpr int kMsWords = 4;           // neighbouring words of a row a lane loads at a time
 
 // Rows of instances of at most kMsMaxN values: 32 rows of one instance at a time by one
 // CTA, their breadth-first searches run together.  Value z has one word each of known,
@@ -319,7 +319,9 @@ constexpr int kMsWords = 4;           // words of a row a lane loads at a time
 // A narrow level costs one L2 round trip (DenseRec) and two barriers: with edge range, edges and
 // queue each read from L2, and a place in the queue taken for each edge, it took 2.9 us, 2.0 now (n =
 // 16,384, out-degree 1.1, 152 levels:
-// 1.74 -> 1.21 ms).
+// 1.74 -> 1.21 ms).  Where searches are short, the rows' matrix words bound it: a lane takes neighbouring
+// words of its row (they share a sector), and a word with no new tuples is not written (n = 16,384,
+// out-degree 0.3: 232 -> 153 us; 2.0: 820 -> 779).
 // Dynamic shared memory: 3 * nmax u32, then the queues: 2 * (gqueue ? kMsNear : nmax) u16.
 constexpr u32 kMsSweep = 64;
 template <int T>
@@ -358,17 +360,17 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
         const bool own = lane < (int)ch.count;
         const u32 n = (u32)d.n;
         const u64 e0 = a.s_csr[d.base], e1 = a.s_csr[min(d.base + d.n, a.rows)];   // the instance's edges
-        for (u32 w0 = warp; w0 < W; w0 += kMsWords * T / 32) {
+        for (u32 w0 = warp * kMsWords; w0 < W; w0 += kMsWords * T / 32) {
             u32 kw[kMsWords], fw[kMsWords];   // the rows' words, in flight together
 #pragma unroll
             for (int u = 0; u < kMsWords; u++) {
-                const u32 w = w0 + u * (T / 32);
+                const u32 w = w0 + u;
                 kw[u] = own && w < W ? krow[w] : 0u;
                 fw[u] = drow != krow && own && w < W ? drow[w] : kw[u];
             }
 #pragma unroll
             for (int u = 0; u < kMsWords; u++) {
-                const u32 w = w0 + u * (T / 32);
+                const u32 w = w0 + u;
                 if (w >= W) break;   // uniform
                 const u32 k = warp_transpose32(kw[u]), f = drow == krow ? k : warp_transpose32(fw[u]);
                 const u32 z = w * 32 + lane;
@@ -497,25 +499,23 @@ __global__ void __launch_bounds__(T) dense_ms_kernel(DenseArgs a, u32 nmax, u16*
         }
         // the rows' new tuples replace their known bits in global memory
         u32 rcnt = 0;
-        for (u32 w0 = warp; w0 < W; w0 += kMsWords * T / 32) {
+        for (u32 w0 = warp * kMsWords; w0 < W; w0 += kMsWords * T / 32) {
             u32 old[kMsWords];
 #pragma unroll
             for (int u = 0; u < kMsWords; u++) {
-                const u32 w = w0 + u * (T / 32);
+                const u32 w = w0 + u;
                 old[u] = own && w < W ? krow[w] : 0u;
             }
 #pragma unroll
             for (int u = 0; u < kMsWords; u++) {
-                const u32 w = w0 + u * (T / 32);
+                const u32 w = w0 + u;
                 if (w >= W) break;
                 const u32 z = w * 32 + lane;
                 const u32 kz = known[z];
                 const u32 nw = warp_transpose32(kz) & ~old[u];
                 if (z < n) relax += row_edges(a, d.base + z) * (u64)__popc(kz);
-                if (own) {
-                    krow[w] = nw;
-                    rcnt += __popc(nw);
-                }
+                if (own && nw != old[u]) krow[w] = nw;
+                if (own) rcnt += __popc(nw);
             }
         }
         if (rcnt) atomicAdd(&s_row[lane], rcnt);
