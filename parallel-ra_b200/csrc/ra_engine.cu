@@ -375,14 +375,14 @@ bool fresh_pages(const void* dst, u64 bytes)
 
 // Device bytes to host memory, complete on return.  A plain copy into fresh pageable memory is
 // bound by the driver's one thread, which takes a page fault for each page it fills; for large
-// reads four threads have the kernel make the pages, in order, 2 MB at a time, while the copy goes on.
-// Measured (16-core host), plain -> so: 45 MB of fresh 4 KB pages 20.5 -> 4.6 ms, of fresh 2 MB ones
-// 9.1 -> 3.5; 12 MB 5.5 -> 2.1 and 2.4 -> 1.9; 8 MB of 2 MB pages 1.7 -> 1.9, so these stay plain.  Six
-// threads meet at the address space's lock (45 MB: 10.9 and 8.1 ms).  Pages that are there already
-// would gain nothing (45 MB: 2.3 ms either way).
+// reads three threads have the kernel make the pages, in order, 1 MB at a time, while the copy goes on.
+// Measured (16-core host), plain -> so: 45 MB of fresh 4 KB pages 20.5 -> 5.2 ms, of fresh 2 MB ones
+// 9.1 -> 4.2; 34 MB of 2 MB pages 3.3 (four threads 3.4, four by 2 MB 3.8); 12 MB 5.5 -> 2.0 and 2.4 -> 1.6;
+// 8 MB of 2 MB pages no faster than plain.  Five threads and more meet at the address space's lock (45 MB:
+// 11.0 and 8.4 ms).  Pages that are there already would gain nothing (45 MB: 2.3 ms either way).
 constexpr u64 kPopulateBytes = 12u << 20;
-constexpr u64 kPopulateBlock = 2u << 20;
-constexpr int kPopulateThreads = 4;
+constexpr u64 kPopulateBlock = 1u << 20;
+constexpr int kPopulateThreads = 3;
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
