@@ -37,7 +37,9 @@ namespace ra {
 
 constexpr int kSpShift = 4;
 constexpr int kSpRows = 1 << kSpShift;   // rows of a tile
-constexpr u32 kSpQueue = 6144;           // tuples of a tile that a warp's own queue holds
+// Tuples of a tile that a warp's own queue holds.  (6,144: a tile of 6,125 in a graph of 2^20 values, whose
+// filter hits in every level, took its warp 1.7 ms, 0.9 and a CTA 0.3 so.)
+constexpr u32 kSpQueue = 4096;
 constexpr u32 kSpBuckets = 1024;         // buckets of four slots of a warp's exact table,
 constexpr u32 kSpTable = 3584;           // and the tuples it holds
 constexpr u32 kSpTry = 4096;             // candidates of a tile, besides two per tuple, that a warp
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__(kSpWarps * 32, kSpCtas) sparse_search_kernel(S
 // in a slot of the table, which keeps the first of them (kSpPending | its thread) until it has its
 // place in the queue.  Bound by the step's chain, an L2 round trip or two and four barriers; a level
 // of a narrow tile takes 2.2 us.  A warp with its queue and an exact table in L2 took 7 ms for
-// 32,768 tuples; n = 70,000, out-degree 1.0 (292 such tiles, given up for their number): 6.1 ms, now 2.8.
+// 32,768 tuples; n = 70,000, out-degree 1.0 (292 such tiles, given up for their number): 6.1 ms, now 1.8.
 constexpr u32 kSpPending = 0x8000u;
 static_assert(kSpBigQueue <= kSpPending && kSpBigThreads <= (int)(kSpNone - kSpPending), "a slot's two meanings");
 static_assert(kSpBigSlots > kSpBigQueue + kSpBigThreads, "a probe meets an empty slot");
