@@ -484,7 +484,7 @@ def run_ours(args, rank, world, local_rank):
         # the timed steps ran the sparse row closure; the instrumented pass keeps the iteration loop
         # (per-launch events), whose join roofline is kept beside it
         moved = 24.0 * st.new_tuples
-        roofline = {"kernel": "sparse_search_kernel + sparse_place_kernel", "bound": "L2 round trips (search), DRAM "
+        roofline = {"kernel": "sparse_search_kernel + sparse_big_kernel + sparse_place_kernel", "bound": "L2 round trips (search), DRAM "
                     "writes scattered over the levels (placement)", "achieved": moved / (st.fixpoint_ms / 1e3) / 1e9,
                     "peak": peak, "unit": "GB/s", "frac": moved / (st.fixpoint_ms / 1e3) / 1e9 / peak,
                     "peak_kind": peak_kind, "traffic": None,

@@ -1454,9 +1454,11 @@ int launch_iteration(ra_program* p, DevScc& d, cudaGraphConditionalHandle cond, 
             b.bs = d.bit[r.out_slot];
             b.bits = p->bits;
             // rows of few words share a tile's look-back, as long as there is a tile for every resident
-            // CTA; wide rows keep a warp each busy.  Measured (1 / 2 / 4 rows per warp): a tree of 2^15
-            // nodes, 1,024 words per row, 8.4 / 8.9 / 9.8 ms; a wave of 96 trees, at most 128 words, 6.2 /
-            // 5.4 / 4.8 ms
+            // CTA; wide rows keep a warp each busy.  Measured, 1 / 2 / 4 / 8 rows per warp and by this rule:
+            // trees of 5,000 values 1.47 / 1.49 / 1.56 / 1.77 and 1.49 ms, of 20,000 4.6 / 4.5 / 5.1 / 5.4 and
+            // 4.6, of 2^15 (1,024 words a row) 8.2 / 8.1 / 8.8 / 10.1 and 8.3; waves of 96 trees of 64 to
+            // 4,096 values 12.3 / 9.3 / 8.0 / 7.6 and 8.0, of 400 of 200 to 1,200 12.7 / 8.6 / 6.7 / 5.9 and 5.8,
+            // of 1,024 of 20 to 80 2.1 / 1.6 / 1.4 / 1.3 and 1.3, of 8 of 6,000 to 9,000 6.9 / 6.1 / 6.0 / 6.2 and 6.1
             const u64 brows = d.bit[r.out_slot].n;
             const u64 bwords = p->n_inst ? p->bmt_total / std::max<u64>(brows, 1) : d.bit[r.out_slot].words;
             b.rows_per_warp = 1;

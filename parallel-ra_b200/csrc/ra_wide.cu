@@ -547,7 +547,7 @@ void wide_iteration(ra_program* p, Scc& s)
             else wide_heads<u64>(p, R, wo.n, wo.cw);
         }
         flush_heads();
-        // membership of the heads in full and delta, one thread per candidate of every relation
+        // membership of the heads in full and delta: a warp per candidate of every relation, or a thread
         WideMemberBatch mb{};
         auto flush_member = [&]() {
             if (!mb.n) return;
