@@ -2823,7 +2823,7 @@ bool run_scc_sparse(ra_program* p, Scc& s)
         CK(cudaMemsetAsync(meta, 0, kMetaWords * 8, p->stream));
         sparse_adj_kernel<<<grid_for(std::max(n, sn)), kThreads, 0, p->stream>>>(a, scsr, sk, sn);
         LAUNCHED();
-        sparse_bounds_kernel<<<grid_for(n_stored + 1), kThreads, 0, p->stream>>>(a);
+        sparse_bounds_kernel<<<grid_for(std::max<u64>(n_stored, a.tiles + 1)), kThreads, 0, p->stream>>>(a);
         LAUNCHED();
         for (int round = 0;; round++) {
             dev_free(p, &B.arena);
