@@ -42,8 +42,9 @@ constexpr int kSpRows = 1 << kSpShift;   // rows of a tile
 constexpr u32 kSpQueue = 4096;
 constexpr u32 kSpBuckets = 1024;         // buckets of four slots of a warp's exact table,
 constexpr u32 kSpTable = 3584;           // and the tuples it holds
-constexpr u32 kSpTry = 4096;             // candidates of a tile, besides two per tuple, that a warp
-constexpr u32 kSpTryMost = 4 * kSpTry;   // takes when there are no other tiles left, and when there are
+constexpr u32 kSpTry = 2048;             // candidates of a tile, besides two per tuple, that a warp
+constexpr u32 kSpTryMost = 16384;        // takes when there are no other tiles left, and when there are;
+constexpr u32 kSpTryOnce = 4096;         // of 32 of its tuples
 constexpr u32 kSpBigQueue = 32768;       // ... and a CTA's, in shared memory
 constexpr u32 kSpBigTry = 262144;
 constexpr u32 kSpBigSlots = 40960;       // slots of a CTA's exact table, beside it
@@ -231,7 +232,7 @@ __device__ __forceinline__ u32 sparse_look(const SparseArgs& a, const u32* q, u3
     }
     if (__shfl_sync(0xffffffffu, stop, 0)) return kSpEndWide;
     if (first && nlv && sparse_grows(a, q, f0, f1, qn, (u32)((1ull << a.bits) - 1))) return kSpEndWide;
-    if (tot > kSpTry || tried > kSpTryMost + 2 * qn) return kSpEndBig;
+    if (tot > kSpTryOnce || tried > kSpTryMost + 2 * qn) return kSpEndBig;
     return __shfl_sync(0xffffffffu, alone, 0) ? kSpEndEarly : 0;
 }
 
