@@ -30,7 +30,9 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <condition_variable>
 #include <functional>
+#include <mutex>
 #include <thread>
 #include <fstream>
 #include <string>
@@ -353,16 +355,18 @@ u64 read_scalar(ra_program* p, const u64* dptr)
     return p->hscalar[0];
 }
 
-// Are pages of the caller's memory still to be made?  (Looks at 16 of them.  No for page-locked,
-// managed and device memory.)
-bool fresh_pages(const void* dst, u64 bytes)
+// Pageable memory of the host (not page-locked, managed or of a device), and are pages of it
+// still to be made (16 of them are looked at)?
+bool pageable(const void* dst)
 {
     cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (at.type != cudaMemoryTypeUnregistered) return false;
+    if (cudaPointerGetAttributes(&at, dst) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
+bool fresh_pages(const void* dst, u64 bytes)
+{
     const u64 page = (u64)sysconf(_SC_PAGESIZE);
     for (u64 i = 0; i < 16; i++) {
         unsigned char here = 1;
@@ -373,26 +377,172 @@ bool fresh_pages(const void* dst, u64 bytes)
     return false;
 }
 
-// Device bytes to host memory, complete on return.  A plain copy into fresh pageable memory is
-// bound by the driver's one thread, which takes a page fault for each page it fills; for large
-// reads three threads have the kernel make the pages, in order, 1 MB at a time, while the copy goes on.
-// Measured (16-core host), plain -> so: 45 MB of fresh 4 KB pages 20.5 -> 5.2 ms, of fresh 2 MB ones
-// 9.1 -> 4.2; 34 MB of 2 MB pages 3.3 (four threads 3.4, four by 2 MB 3.8); 12 MB 5.5 -> 2.0 and 2.4 -> 1.6;
-// 8 MB of 2 MB pages no faster than plain.  Five threads and more meet at the address space's lock (45 MB:
-// 11.0 and 8.4 ms).  Pages that are there already would gain nothing (45 MB: 2.3 ms either way).
+// Device bytes to host memory, complete on return.  A plain copy into pageable memory is bound by
+// the driver's one thread, which moves staged bytes on and takes a page fault for each fresh page it
+// fills.  Page-locked, managed and device memory, and reads below kPopulateBytes, get that copy.
+//
+// Into fresh pages, three threads have the kernel make the pages, in order, 1 MB at a time, while
+// the copy goes on.  Measured (16-core host), plain -> so: 45 MB of fresh 4 KB pages 20.5 -> 5.2 ms, of
+// fresh 2 MB ones 9.1 -> 4.2; 34 MB of 2 MB pages 3.3 (four threads 3.4, four by 2 MB 3.8); 12 MB 5.5 -> 2.0
+// and 2.4 -> 1.6; 8 MB of 2 MB pages no faster than plain.  Five threads and more meet at the address
+// space's lock (45 MB: 11.0 and 8.4 ms).
+//
+// A process that goes on reading kRingBytes or more gets a page-locked ring of 12 MB, which the copies
+// land in and four threads move on: 45 MB of touched pages 2.3 -> 1.9 ms, 100 MB 5.0 -> 3.2 to 4.3; 20 MB
+// no faster.  It costs 2.5 ms (7 to 12 without huge pages), so it is made by the kRingReads-th such read
+// since the process's programs came into being, and goes with the last of them: programs made for one read
+// never pay for it.  One read uses it at a time; another one meanwhile goes without.
 constexpr u64 kPopulateBytes = 12u << 20;
 constexpr u64 kPopulateBlock = 1u << 20;
 constexpr int kPopulateThreads = 3;
+constexpr u64 kRingBytes = 24u << 20;
+constexpr int kRingReads = 4;
+constexpr u64 kRingChunk = 2u << 20;
+constexpr int kRingChunks = 6;
+constexpr int kRingThreads = 4;
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
 
+struct HostRing {
+    std::mutex busy;          // held while a read uses, makes or frees the buffer
+    std::mutex count_mu;
+    int programs = 0;
+    int reads = 0;
+    char *map = nullptr, *buf = nullptr;
+    void add()
+    {
+        std::lock_guard<std::mutex> lk(count_mu);
+        programs++;
+    }
+    void remove()
+    {
+        std::lock_guard<std::mutex> lk(count_mu);
+        if (--programs) return;
+        std::lock_guard<std::mutex> use(busy);
+        reads = 0;
+        drop();
+    }
+    // with `busy` held: the buffer, made by now or not
+    char* get()
+    {
+        if (buf || reads < 0 || ++reads < kRingReads) return buf;
+        reads = -1;   // one attempt
+        void* q = mmap(nullptr, kRingChunk * (kRingChunks + 1), PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        if (q == MAP_FAILED) return nullptr;
+        map = (char*)q;
+        char* at = (char*)(((u64)map + kRingChunk - 1) & ~(kRingChunk - 1));   // whole huge pages
+        madvise(at, kRingChunk * kRingChunks, MADV_HUGEPAGE);
+        if (cudaHostRegister(at, kRingChunk * kRingChunks, cudaHostRegisterPortable) == cudaSuccess) {
+            buf = at;
+        } else {
+            cudaGetLastError();
+            drop();
+        }
+        return buf;
+    }
+    void drop()
+    {
+        if (buf) cudaHostUnregister(buf);
+        if (map) munmap(map, kRingChunk * (kRingChunks + 1));
+        map = buf = nullptr;
+    }
+};
+HostRing g_ring;
+
+// The read through the ring, by chunks; kRingThreads threads (or this one, if none can be had) move them on.
+void rows_through_ring(ra_program* p, char* buf, void* dst, const void* src, u64 bytes)
+{
+    struct Events {
+        cudaEvent_t e[kRingChunks] = {};
+        ~Events()
+        {
+            for (cudaEvent_t v : e)
+                if (v) cudaEventDestroy(v);
+        }
+    } ev;
+    for (cudaEvent_t& e : ev.e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const u64 chunks = (bytes + kRingChunk - 1) / kRingChunk;
+    auto move_on = [&](u64 i) {
+        const u64 at = i * kRingChunk;
+        std::memcpy((char*)dst + at, buf + (i % kRingChunks) * kRingChunk, std::min(kRingChunk, bytes - at));
+    };
+    std::vector<char> moved(chunks, 0);
+    std::mutex mu;
+    std::condition_variable more, room;   // a chunk landed (or the read ended); a chunk was moved on
+    u64 ready = 0, taken = 0;             // chunks landed, chunks a thread has taken
+    bool end = false;
+    auto work = [&]() {
+        std::unique_lock<std::mutex> lk(mu);
+        for (;;) {
+            more.wait(lk, [&] { return end || taken < ready; });
+            if (taken >= ready) return;
+            const u64 i = taken++;
+            lk.unlock();
+            move_on(i);
+            lk.lock();
+            moved[i] = 1;
+            room.notify_one();
+        }
+    };
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(kRingThreads);
+        for (int t = 0; t < kRingThreads; t++) pool.emplace_back(work);
+    } catch (...) {   // as many threads as could be had; none: this one moves the chunks
+    }
+    cudaError_t err = cudaSuccess;
+    u64 issued = 0;
+    for (u64 landed = 0; landed < chunks && err == cudaSuccess; landed++) {
+        while (issued < chunks && issued < landed + kRingChunks && err == cudaSuccess) {
+            if (issued >= (u64)kRingChunks && !pool.empty()) {   // its slot's last chunk must have left
+                std::unique_lock<std::mutex> lk(mu);
+                const u64 old = issued - kRingChunks;
+                if (issued > landed && !moved[old]) break;   // other chunks are in flight: see to those
+                room.wait(lk, [&] { return moved[old] != 0; });
+            }
+            const u64 at = issued * kRingChunk, slot = issued % kRingChunks;
+            err = cudaMemcpyAsync(buf + slot * kRingChunk, (const char*)src + at, std::min(kRingChunk, bytes - at),
+                                  cudaMemcpyDeviceToHost, p->stream);
+            if (err == cudaSuccess) err = cudaEventRecord(ev.e[slot], p->stream);
+            issued++;
+        }
+        if (err == cudaSuccess) err = cudaEventSynchronize(ev.e[landed % kRingChunks]);
+        if (err != cudaSuccess) break;
+        if (pool.empty()) {
+            move_on(landed);
+            continue;
+        }
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            ready = landed + 1;
+        }
+        more.notify_one();
+    }
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        end = true;
+    }
+    more.notify_all();
+    for (std::thread& t : pool) t.join();
+    if (err != cudaSuccess) cudaStreamSynchronize(p->stream);   // no copy still writes the ring
+    ck(p, err, "rows to host");
+}
+
 void rows_to_host(ra_program* p, void* dst, const void* src, u64 bytes)
 {
+    const bool threads = bytes >= kPopulateBytes && std::thread::hardware_concurrency() >= 2 * kRingThreads && pageable(dst);
+    if (threads && bytes >= kRingBytes) {
+        std::unique_lock<std::mutex> use(g_ring.busy, std::try_to_lock);
+        char* buf = use ? g_ring.get() : nullptr;
+        if (buf) {
+            rows_through_ring(p, buf, dst, src, bytes);
+            return;
+        }
+    }
     std::vector<std::thread> pool;
     std::atomic<u64> next{0};
-    if (bytes >= kPopulateBytes && std::thread::hardware_concurrency() >= 2 * kPopulateThreads &&
-        fresh_pages(dst, bytes)) {
+    if (threads && fresh_pages(dst, bytes)) {
         const u64 page = (u64)sysconf(_SC_PAGESIZE);
         const u64 first = ((u64)dst + page - 1) & ~(page - 1), last = ((u64)dst + bytes) & ~(page - 1);
         try {
@@ -3574,6 +3724,7 @@ int ra_program_create(int device, ra_program** out)
         delete p;
         return st;
     }
+    g_ring.add();
     *out = p;
     return RA_OK;
 }
@@ -3643,6 +3794,7 @@ int ra_program_destroy(ra_program* p)
     }
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
+    g_ring.remove();
     return RA_OK;
 }
 

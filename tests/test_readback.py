@@ -1,5 +1,5 @@
 """Rows read back to host memory: by one copy, into large fresh memory (12 MB up) while several
-threads make its pages; every size gives the loaded rows in trie order."""
+threads make its pages, or through a ring; every size gives the loaded rows in trie order."""
 import ctypes as C
 import mmap
 import threading
@@ -137,3 +137,31 @@ def test_a_program_s_first_read_costs_no_set_up():
         again += [read_into(p, r, at, len(want)) for _ in range(3)]
         p.close()
     assert min(first) < 2 * min(again) + 1e-3
+
+
+def test_a_process_that_goes_on_reading():
+    """From the fourth read of 24 MB or more on through a ring, made with the reads and given back with
+    the last program: whole, odd and partial chunks, several programs, then all closed and again."""
+    for _ in range(2):
+        progs = [loaded(n) for n in (12 * CHUNK, 12 * CHUNK + 24, 13 * CHUNK - 24, 20 * CHUNK + 24)]
+        for k in range(3):
+            for p, r, want in progs:
+                assert np.array_equal(p.dump_full(r), want), k
+        at, keep = mapped(progs[3][2].nbytes, "some touched")
+        for p, r, want in progs:
+            read_into(p, r, at, len(want))
+            assert np.array_equal(np.ctypeslib.as_array(C.cast(at, C.POINTER(C.c_uint64)), want.shape), want)
+        for p, r, want in progs:
+            p.close()
+
+
+def test_a_program_s_first_large_read_costs_no_ring():
+    """Programs made for one read of 30 MB, one after the other: no read pays for a ring."""
+    at, keep = mapped(31 << 20, "all touched")
+    first, plain = [], []
+    for k in range(8):
+        p, r, want = loaded(30 << 20)
+        first.append(read_into(p, r, at, len(want)))
+        plain += [read_into(p, r, at, len(want)) for _ in range(2)]   # the second and third read: none yet
+        p.close()
+    assert np.median(first) < 1.5 * np.median(plain) + 1e-3
